@@ -44,6 +44,24 @@ class RmiError(RuntimeError):
         self.message = message
 
 
+# Argument types of the entry points that a token loop calls: with them ctypes takes plain integers for pointers and
+# sizes, which costs a third of wrapping every argument in an object of its own.
+_V, _N, _I = C.c_void_p, C.c_size_t, C.c_int32
+_PROTOTYPES = {
+    "rmi_matmul_q8_0": [_V, _V, _V, _N, _V],
+    "rmi_matmul_q8_0_dev": [_V, _V, _V, _N, _V],
+    "rmi_matmul_q8_0_dev_noalloc": [_V, _V, _V, _N, _V],
+    "rmi_matmul_q8_0_f32_dev": [_V, _V, _V, _N, _V],
+    "rmi_matmul_q8_0_prequantized_dev": [_V, _V, _V, _V, _N, _V, _N, _N],
+    "rmi_ffn_swiglu_q8_0_dev": [_V, _V, _V, _V, _N, _V],
+    "rmi_quantize_q8_0_dev": [_V, _V, _N, _N, _V, _V],
+    "rmi_matmul_q4_k_q8k": [_V, _V, _V, _N, _V, _N, _N],
+    "rmi_matmul_q4_k_q8k_dev": [_V, _V, _V, _N, _V],
+    "rmi_matmul_q4_k_dequant_dev": [_V, _V, _V, _N, _V],
+    "rmi_matmul_q6_k_q8k": [_V, _V, _V, _N, _V, _N, _N],
+    "rmi_matmul_q4_0": [_V, _V, _V, _N, _V],
+    "rmi_session_step": [_V, _V, _V, _V, _V],
+}
 _lib = None
 
 
@@ -55,6 +73,8 @@ def lib() -> C.CDLL:
             raise RuntimeError(f"{LIB_PATH} is missing: run `python __graft_entry__.py build` first")
         _lib = C.CDLL(LIB_PATH)
         _lib.rmi_last_error.restype = C.c_char_p
+        for name, types in _PROTOTYPES.items():
+            getattr(_lib, name).argtypes = types
     return _lib
 
 
@@ -296,7 +316,33 @@ class Kernel:
             self.forward(input[t * n_in:(t + 1) * n_in], output.reshape(-1)[t * n_out:(t + 1) * n_out], n_in, n_out)
 
 
-class Q8Kernel(Kernel):
+class _DeviceKernel(Kernel):
+    """`forward` and `forward_batched` as one device call each: the activation is quantized there, which gives the bytes
+    of quantize_q8_0_into (the quantizers are deterministic), and all tokens share the pass over the weight."""
+
+    def _forward_rows(self, x: int, m: int, out: int):
+        """m rows at host address x -> m rows of all n_out outputs at host address out"""
+        raise NotImplementedError
+
+    def forward(self, input, output, n_in, n_out):
+        input = np.ascontiguousarray(input, np.float32)
+        if n_in != self.weight.n_in or n_out != self.weight.n_out or input.size != n_in:
+            return super().forward(input, output, n_in, n_out)  # fewer outputs than the weight has
+        assert output.dtype == np.float32 and output.flags.c_contiguous and output.size >= n_out
+        self._forward_rows(input.ctypes.data, 1, output.ctypes.data)
+
+    def forward_batched(self, input, output, n_in, n_out):
+        input = np.ascontiguousarray(input, np.float32)
+        n_tokens = input.size // n_in
+        if n_in != self.weight.n_in or n_out != self.weight.n_out:
+            return super().forward_batched(input, output, n_in, n_out)
+        assert input.size == n_tokens * n_in and output.size == n_tokens * n_out
+        assert output.dtype == np.float32 and output.flags.c_contiguous
+        if n_tokens:
+            self._forward_rows(input.ctypes.data, n_tokens, output.ctypes.data)
+
+
+class Q8Kernel(_DeviceKernel):
     """Q8Kernel (src/ops/kernel/q8_0/mod.rs:22-56)."""
 
     @classmethod
@@ -306,20 +352,20 @@ class Q8Kernel(Kernel):
     def forward_prequantized(self, input_q8, input_scales, output, n_in, n_out, ith, nth):
         matmul_q8_0_quantized_parallel_rows(self.weight, input_q8, input_scales, output, n_in, n_out, ith, nth)
 
-    def forward_batched(self, input, output, n_in, n_out):
-        """One call for all tokens: rmi_matmul_q8_0 quantizes row-wise and picks GEMV or GEMM."""
-        input = np.ascontiguousarray(input, np.float32).reshape(-1, n_in)
-        assert output.dtype == np.float32 and output.flags.c_contiguous and output.size == input.shape[0] * n_out
-        assert n_in == self.weight.n_in and n_out == self.weight.n_out
-        _check(lib().rmi_matmul_q8_0(self._ctx.handle, self.weight._h, _p(input), _sz(input.shape[0]), _p(output)))
+    def _forward_rows(self, x, m, out):
+        # quantizes row-wise and picks GEMV or GEMM
+        _check(lib().rmi_matmul_q8_0(self._ctx.handle, self.weight._h, x, m, out))
 
 
-class Q4_KKernel(Kernel):
+class Q4_KKernel(_DeviceKernel):
     """Q4_KKernel (src/ops/kernel/q4_k.rs:7-93)."""
 
     @classmethod
     def new(cls, data, n_in: int, n_out: int, ctx: Context | None = None) -> "Q4_KKernel":
         return cls(QuantizedTensor.from_bytes(data, GGML_Q4_K, n_in, n_out, ctx=ctx))
+
+    def _forward_rows(self, x, m, out):
+        _check(lib().rmi_matmul_q4_k_q8k(self._ctx.handle, self.weight._h, x, m, out, 0, self.weight.n_out))
 
     def forward_prepared(self, input_f32, input_q8, input_scales, q8_k, output, n_in, n_out, ith, nth):
         # q4_k.rs:56-93; a caller-prepared Q8_K (q8_k) is recomputed on the device from input_f32,
@@ -347,12 +393,15 @@ class Q4_KKernel(Kernel):
         output.reshape(-1)[s:e] = full[s:e]
 
 
-class Q6_KKernel(Kernel):
+class Q6_KKernel(_DeviceKernel):
     """Q6_KKernel (src/ops/kernel/q6_k.rs:7-80)."""
 
     @classmethod
     def new(cls, data, n_in: int, n_out: int, ctx: Context | None = None) -> "Q6_KKernel":
         return cls(QuantizedTensor.from_bytes(data, GGML_Q6_K, n_in, n_out, ctx=ctx))
+
+    def _forward_rows(self, x, m, out):
+        _check(lib().rmi_matmul_q6_k_q8k(self._ctx.handle, self.weight._h, x, m, out, 0, self.weight.n_out))
 
     def forward_prepared(self, input_f32, input_q8, input_scales, q8_k, output, n_in, n_out, ith, nth):
         # q6_k.rs:44-80; a caller-prepared Q8_K is recomputed on the device from input_f32 (deterministic)
@@ -376,12 +425,15 @@ class Q6_KKernel(Kernel):
                                                   _sz(s), _sz(e)))
 
 
-class Q4_0Kernel(Kernel):
+class Q4_0Kernel(_DeviceKernel):
     """Q4_0Kernel (src/ops/kernel/q4_0/mod.rs:14-80)."""
 
     @classmethod
     def new(cls, data, n_in: int, n_out: int, ctx: Context | None = None) -> "Q4_0Kernel":
         return cls(QuantizedTensor.from_bytes(data, GGML_Q4_0, n_in, n_out, ctx=ctx))
+
+    def _forward_rows(self, x, m, out):
+        _check(lib().rmi_matmul_q4_0(self._ctx.handle, self.weight._h, x, m, out))
 
     def forward_prequantized(self, input_q8, input_scales, output, n_in, n_out, ith, nth):
         q8 = np.ascontiguousarray(input_q8, np.uint8).reshape(-1)[:n_in]
@@ -501,7 +553,7 @@ def matmul_q8_0_f32(weight: QuantizedTensor, x) -> np.ndarray:
 
 
 def matmul_q8_0_f32_dev(weight: QuantizedTensor, x_ptr: int, m: int, out_ptr: int):
-    _check(lib().rmi_matmul_q8_0_f32_dev(weight._ctx.handle, weight._h, C.c_void_p(x_ptr), _sz(m), C.c_void_p(out_ptr)))
+    _check(lib().rmi_matmul_q8_0_f32_dev(weight._ctx._h, weight._h, x_ptr, m, out_ptr))
 
 
 def q8_0_block_sums(weight: QuantizedTensor, q8, m: int, use_tensor_cores: bool = False) -> np.ndarray:
@@ -547,40 +599,34 @@ def ffn_swiglu_q8_0_pipelined(w_gate_up, w_down, x_ptrs, out_ptrs, m: int):
 # torch.Tensor.data_ptr() or Context.dev_alloc().
 
 def ffn_swiglu_q8_0_dev(w_gate_up: QuantizedTensor, w_down: QuantizedTensor, x_ptr: int, m: int, out_ptr: int):
-    _check(lib().rmi_ffn_swiglu_q8_0_dev(w_gate_up._ctx.handle, w_gate_up._h, w_down._h, C.c_void_p(x_ptr), _sz(m),
-                                         C.c_void_p(out_ptr)))
+    _check(lib().rmi_ffn_swiglu_q8_0_dev(w_gate_up._ctx._h, w_gate_up._h, w_down._h, x_ptr, m, out_ptr))
 
 
 def matmul_q8_0_dev(weight: QuantizedTensor, x_ptr: int, m: int, out_ptr: int):
-    _check(lib().rmi_matmul_q8_0_dev(weight._ctx.handle, weight._h, C.c_void_p(x_ptr), _sz(m), C.c_void_p(out_ptr)))
+    _check(lib().rmi_matmul_q8_0_dev(weight._ctx._h, weight._h, x_ptr, m, out_ptr))
 
 
 def matmul_q8_0_dev_noalloc(weight: QuantizedTensor, x_ptr: int, m: int, out_ptr: int):
     """Allocation-free variant of matmul_q8_0_dev (m <= 32, m * n_in <= 524288): see include/rmi_cuda.h."""
-    _check(lib().rmi_matmul_q8_0_dev_noalloc(weight._ctx.handle, weight._h, C.c_void_p(x_ptr), _sz(m),
-                                             C.c_void_p(out_ptr)))
+    _check(lib().rmi_matmul_q8_0_dev_noalloc(weight._ctx._h, weight._h, x_ptr, m, out_ptr))
 
 
 def matmul_q8_0_prequantized_dev(weight: QuantizedTensor, q8_ptr: int, scales_ptr: int, m: int, out_ptr: int,
                                  row_begin: int = 0, row_end: int | None = None):
     row_end = weight.n_out if row_end is None else row_end
-    _check(lib().rmi_matmul_q8_0_prequantized_dev(weight._ctx.handle, weight._h, C.c_void_p(q8_ptr),
-                                                  C.c_void_p(scales_ptr), _sz(m), C.c_void_p(out_ptr), _sz(row_begin),
-                                                  _sz(row_end)))
+    _check(lib().rmi_matmul_q8_0_prequantized_dev(weight._ctx._h, weight._h, q8_ptr, scales_ptr, m, out_ptr, row_begin, row_end))
 
 
 def quantize_q8_0_dev(ctx: Context, x_ptr: int, m: int, n: int, q8_ptr: int, scales_ptr: int):
-    _check(lib().rmi_quantize_q8_0_dev(ctx.handle, C.c_void_p(x_ptr), _sz(m), _sz(n), C.c_void_p(q8_ptr),
-                                       C.c_void_p(scales_ptr)))
+    _check(lib().rmi_quantize_q8_0_dev(ctx._h, x_ptr, m, n, q8_ptr, scales_ptr))
 
 
 def matmul_q4_k_q8k_dev(weight: QuantizedTensor, x_ptr: int, m: int, out_ptr: int):
-    _check(lib().rmi_matmul_q4_k_q8k_dev(weight._ctx.handle, weight._h, C.c_void_p(x_ptr), _sz(m), C.c_void_p(out_ptr)))
+    _check(lib().rmi_matmul_q4_k_q8k_dev(weight._ctx._h, weight._h, x_ptr, m, out_ptr))
 
 
 def matmul_q4_k_dequant_dev(weight: QuantizedTensor, x_ptr: int, m: int, out_ptr: int):
-    _check(lib().rmi_matmul_q4_k_dequant_dev(weight._ctx.handle, weight._h, C.c_void_p(x_ptr), _sz(m),
-                                             C.c_void_p(out_ptr)))
+    _check(lib().rmi_matmul_q4_k_dequant_dev(weight._ctx._h, weight._h, x_ptr, m, out_ptr))
 
 
 def unshard_cols_dev(ctx: Context, gathered_ptr: int, g: int, m: int, n_per_rank: int, out_ptr: int):

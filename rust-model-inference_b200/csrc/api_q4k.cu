@@ -41,18 +41,14 @@ extern "C" int32_t rmi_matmul_q4_k_q8k(rmi_ctx* ctx, const rmi_weight* w, const 
   float *dx, *dd, *dout;
   int8_t* dq;
   int16_t* db;
-  RMI_TRY(rmi_scratch(ctx, 5, m * n * 4, (void**)&dx));
+  RMI_TRY(host_in(ctx, x, m * n * 4, 5, true, (void**)&dx));
   RMI_TRY(rmi_scratch(ctx, 0, m * n, (void**)&dq));
   RMI_TRY(rmi_scratch(ctx, 1, nb * 4, (void**)&dd));
   RMI_TRY(rmi_scratch(ctx, 4, nb * 32, (void**)&db));
   RMI_TRY(rmi_scratch(ctx, 6, m * w->n_rows * 4, (void**)&dout));
-  RMI_CUDA_CHECK(cudaMemcpyAsync(dx, x, m * n * 4, cudaMemcpyHostToDevice, ctx->stream));
   RMI_TRY(launch_q8k_quantize(ctx, dx, m, n, dd, dq, db));
   RMI_TRY(launch_q4k_q8k_matmul(ctx, w, dd, dq, db, m, dout, row_begin, row_end));
-  RMI_CUDA_CHECK(cudaMemcpy2DAsync(output + row_begin, w->n_rows * 4, dout + row_begin, w->n_rows * 4, nr * 4, m,
-                                   cudaMemcpyDeviceToHost, ctx->stream));
-  RMI_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
-  return RMI_OK;
+  return host_out(ctx, output + row_begin, dout + row_begin, m, nr * 4, w->n_rows * 4);
 }
 
 extern "C" int32_t rmi_matmul_q4_k_q8k_dev(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, float* output) {
@@ -88,13 +84,10 @@ extern "C" int32_t rmi_matmul_q4_k_dequant(rmi_ctx* ctx, const rmi_weight* w, co
   RMI_REQUIRE(x && output, RMI_ERR_BAD_HANDLE, "rmi_matmul_q4_k_dequant: null buffer");
   std::lock_guard<std::mutex> lock(ctx->mu);
   float *dx, *dout;
-  RMI_TRY(rmi_scratch(ctx, 5, m * w->n_in * 4, (void**)&dx));
+  RMI_TRY(host_in(ctx, x, m * w->n_in * 4, 5, false, (void**)&dx));
   RMI_TRY(rmi_scratch(ctx, 6, m * w->n_rows * 4, (void**)&dout));
-  RMI_CUDA_CHECK(cudaMemcpyAsync(dx, x, m * w->n_in * 4, cudaMemcpyHostToDevice, ctx->stream));
   RMI_TRY(launch_q4k_dequant_matmul(ctx, w, dx, m, dout));
-  RMI_CUDA_CHECK(cudaMemcpyAsync(output, dout, m * w->n_rows * 4, cudaMemcpyDeviceToHost, ctx->stream));
-  RMI_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
-  return RMI_OK;
+  return host_out(ctx, output, dout, 1, m * w->n_rows * 4, 0);
 }
 
 extern "C" int32_t rmi_dequantize_q4_k(rmi_ctx* ctx, const rmi_weight* w, float* output) {
@@ -127,18 +120,14 @@ extern "C" int32_t rmi_matmul_q6_k_q8k(rmi_ctx* ctx, const rmi_weight* w, const 
   float *dx, *dd, *dout;
   int8_t* dq;
   int16_t* db;
-  RMI_TRY(rmi_scratch(ctx, 5, m * n * 4, (void**)&dx));
+  RMI_TRY(host_in(ctx, x, m * n * 4, 5, true, (void**)&dx));
   RMI_TRY(rmi_scratch(ctx, 0, m * n, (void**)&dq));
   RMI_TRY(rmi_scratch(ctx, 1, nb * 4, (void**)&dd));
   RMI_TRY(rmi_scratch(ctx, 4, nb * 32, (void**)&db));
   RMI_TRY(rmi_scratch(ctx, 6, m * w->n_rows * 4, (void**)&dout));
-  RMI_CUDA_CHECK(cudaMemcpyAsync(dx, x, m * n * 4, cudaMemcpyHostToDevice, ctx->stream));
   RMI_TRY(launch_q8k_quantize(ctx, dx, m, n, dd, dq, db));
   RMI_TRY(launch_q6k_q8k_matmul(ctx, w, dd, dq, db, m, dout, row_begin, row_end));
-  RMI_CUDA_CHECK(cudaMemcpy2DAsync(output + row_begin, w->n_rows * 4, dout + row_begin, w->n_rows * 4, nr * 4, m,
-                                   cudaMemcpyDeviceToHost, ctx->stream));
-  RMI_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
-  return RMI_OK;
+  return host_out(ctx, output + row_begin, dout + row_begin, m, nr * 4, w->n_rows * 4);
 }
 
 extern "C" int32_t rmi_matmul_q6_k_prequantized(rmi_ctx* ctx, const rmi_weight* w, const uint8_t* q8, const float* scales,
@@ -153,16 +142,12 @@ extern "C" int32_t rmi_matmul_q6_k_prequantized(rmi_ctx* ctx, const rmi_weight* 
   const size_t n = w->n_in, nr = row_end - row_begin;
   uint8_t* dq;
   float *ds, *dout;
-  RMI_TRY(rmi_scratch(ctx, 0, m * n, (void**)&dq));
+  RMI_TRY(host_in(ctx, q8, m * n, 0, false, (void**)&dq));
   RMI_TRY(rmi_scratch(ctx, 1, m * (n / 32) * 4, (void**)&ds));
   RMI_TRY(rmi_scratch(ctx, 6, m * w->n_rows * 4, (void**)&dout));
-  RMI_CUDA_CHECK(cudaMemcpyAsync(dq, q8, m * n, cudaMemcpyHostToDevice, ctx->stream));
   RMI_CUDA_CHECK(cudaMemcpyAsync(ds, scales, m * (n / 32) * 4, cudaMemcpyHostToDevice, ctx->stream));
   RMI_TRY(launch_q6k_prequant_matmul(ctx, w, dq, ds, m, dout, row_begin, row_end));
-  RMI_CUDA_CHECK(cudaMemcpy2DAsync(output + row_begin, w->n_rows * 4, dout + row_begin, w->n_rows * 4, nr * 4, m,
-                                   cudaMemcpyDeviceToHost, ctx->stream));
-  RMI_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
-  return RMI_OK;
+  return host_out(ctx, output + row_begin, dout + row_begin, m, nr * 4, w->n_rows * 4);
 }
 
 extern "C" int32_t rmi_dequantize_q6_k(rmi_ctx* ctx, const rmi_weight* w, float* output) {
@@ -193,16 +178,12 @@ extern "C" int32_t rmi_matmul_q4_0_prequantized(rmi_ctx* ctx, const rmi_weight* 
   const size_t n = w->n_in, nr = row_end - row_begin;
   uint8_t* dq;
   float *ds, *dout;
-  RMI_TRY(rmi_scratch(ctx, 0, m * n, (void**)&dq));
+  RMI_TRY(host_in(ctx, q8, m * n, 0, false, (void**)&dq));
   RMI_TRY(rmi_scratch(ctx, 1, m * (n / 32) * 4, (void**)&ds));
   RMI_TRY(rmi_scratch(ctx, 6, m * w->n_rows * 4, (void**)&dout));
-  RMI_CUDA_CHECK(cudaMemcpyAsync(dq, q8, m * n, cudaMemcpyHostToDevice, ctx->stream));
   RMI_CUDA_CHECK(cudaMemcpyAsync(ds, scales, m * (n / 32) * 4, cudaMemcpyHostToDevice, ctx->stream));
   RMI_TRY(launch_q4_0_matmul(ctx, w, dq, ds, m, dout, row_begin, row_end));
-  RMI_CUDA_CHECK(cudaMemcpy2DAsync(output + row_begin, w->n_rows * 4, dout + row_begin, w->n_rows * 4, nr * 4, m,
-                                   cudaMemcpyDeviceToHost, ctx->stream));
-  RMI_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
-  return RMI_OK;
+  return host_out(ctx, output + row_begin, dout + row_begin, m, nr * 4, w->n_rows * 4);
 }
 
 extern "C" int32_t rmi_matmul_q4_0(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, float* output) {
@@ -214,16 +195,13 @@ extern "C" int32_t rmi_matmul_q4_0(rmi_ctx* ctx, const rmi_weight* w, const floa
   const size_t n = w->n_in;
   uint8_t* dq;
   float *dx, *ds, *dout;
-  RMI_TRY(rmi_scratch(ctx, 5, m * n * 4, (void**)&dx));
+  RMI_TRY(host_in(ctx, x, m * n * 4, 5, true, (void**)&dx));
   RMI_TRY(rmi_scratch(ctx, 0, m * n, (void**)&dq));
   RMI_TRY(rmi_scratch(ctx, 1, m * (n / 32) * 4, (void**)&ds));
   RMI_TRY(rmi_scratch(ctx, 6, m * w->n_rows * 4, (void**)&dout));
-  RMI_CUDA_CHECK(cudaMemcpyAsync(dx, x, m * n * 4, cudaMemcpyHostToDevice, ctx->stream));
   RMI_TRY(launch_q8_quantize(ctx, dx, m, n, dq, ds, 0));
   RMI_TRY(launch_q4_0_matmul(ctx, w, dq, ds, m, dout, 0, w->n_rows));
-  RMI_CUDA_CHECK(cudaMemcpyAsync(output, dout, m * w->n_rows * 4, cudaMemcpyDeviceToHost, ctx->stream));
-  RMI_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
-  return RMI_OK;
+  return host_out(ctx, output, dout, 1, m * w->n_rows * 4, 0);
 }
 
 // ---------------------------------------------------------------- embedding lookup

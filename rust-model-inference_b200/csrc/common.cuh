@@ -102,6 +102,9 @@ struct rmi_ctx {
   cudaStream_t copy_in, copy_out;
   cudaEvent_t ev_in[2], ev_compute[2], ev_out[2];
   bool pipe_ready;
+  // pinned staging of the host-pointer entry points (host_in / host_out), created on first use
+  uint8_t *pin_in, *pin_out;   // host addresses
+  uint8_t *pin_in_dev;         // device address of pin_in
 };
 
 // Q8_0 / Q4_K weight resident in HBM.
@@ -143,6 +146,11 @@ int32_t rmi_check_ctx(rmi_ctx* ctx);
 int32_t rmi_check_weight(const rmi_weight* w, int ggml_type);
 int32_t rmi_scratch(rmi_ctx* ctx, int slot, size_t bytes, void** out);
 int32_t rmi_post_launch(rmi_ctx* ctx, const char* what);
+// Host-pointer entry points.  host_in: makes `bytes` of host memory readable by the next kernel (scratch slot `slot` or
+// the mapped staging buffer; `once`: the kernel reads every byte once).  host_out: copies rows of a device buffer back,
+// synchronising the stream; rows x row_bytes with `pitch` bytes from row to row on both sides.  One of each per call.
+int32_t host_in(rmi_ctx* ctx, const void* src, size_t bytes, int slot, bool once, void** dev);
+int32_t host_out(rmi_ctx* ctx, void* dst, const void* src, size_t rows, size_t row_bytes, size_t pitch);
 int32_t rmi_check_dev_status(rmi_ctx* ctx, const char* what);
 // Returns a record index (or -1 when timing is off); pass it to rmi_prof_end after the launch.
 int rmi_prof_begin(rmi_ctx* ctx, const char* tag);
@@ -177,6 +185,25 @@ static inline cudaError_t rmi_launch(const rmi_ctx* ctx, void (*kern)(KArgs...),
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
+// The second kernel of a pair enqueued by one call (quantizer -> matmul): always a programmatic dependent, so its
+// set-up and weight copies overlap the first kernel.  The first one of the next call is launched plainly and waits for
+// all of this one; the kernel must call pdl_wait() as above.
+template <typename... KArgs, typename... Args>
+static inline cudaError_t rmi_launch_after(const rmi_ctx* ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                           Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
 // One f32 result to the primary output and to every extra copy.
 __device__ __forceinline__ void store_fanout(float* o, float v, const out_fanout& fo) {
   *o = v;
@@ -206,6 +233,29 @@ __device__ __forceinline__ float exp_cr(float x) { return (float)exp((double)x);
 // adding a small integer to its bit pattern stays exact.
 __device__ __forceinline__ float small_int_to_f32(int v) {
   return __fsub_rn(__int_as_float(v + 0x4B400000), 12582912.0f);
+}
+
+// Bounded wait on a shared-memory mbarrier phase; false when the limit ran out.
+__device__ __forceinline__ bool mbar_wait_limited(uint32_t bar, uint32_t parity, uint64_t limit_ns) {
+  uint64_t t0 = 0;
+  for (uint32_t i = 0; i < (1u << 26); i++) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity), "r"(20000u)
+        : "memory");
+    if (ok) return true;
+    if ((i & 15) == 15) {
+      uint64_t now;
+      asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > limit_ns) return false;
+    }
+  }
+  return false;
 }
 
 __device__ __forceinline__ int dp4a_s8(int a, int b, int c) { return __dp4a(a, b, c); }

@@ -426,29 +426,6 @@ __host__ __device__ inline size_t q4s_smem_bytes(size_t mb, size_t nb) {
   return (size_t)Q4S_RING_BYTES + 128 + mb * nb * (256 + 32 + 4);
 }
 
-// Bounded wait on a shared-memory mbarrier phase; false when the limit ran out.
-__device__ __forceinline__ bool mbar_wait_limited(uint32_t bar, uint32_t parity, uint64_t limit_ns) {
-  uint64_t t0 = 0;
-  for (uint32_t i = 0; i < (1u << 26); i++) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity), "r"(20000u)
-        : "memory");
-    if (ok) return true;
-    if ((i & 15) == 15) {
-      uint64_t now;
-      asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
-      if (t0 == 0) t0 = now;
-      else if (now - t0 > limit_ns) return false;
-    }
-  }
-  return false;
-}
-
 template <int MB>
 __global__ void __launch_bounds__(32 * Q4S_WARPS)
     q4k_q8k_stream_kernel(const uint8_t* __restrict__ w, size_t nb, size_t n_rows, const float* __restrict__ d8,
@@ -493,6 +470,7 @@ __global__ void __launch_bounds__(32 * Q4S_WARPS)
   }
   __syncwarp();
   for (size_t j = 0; j < n_items && j < (size_t)Q4S_S; j++) issue(j);
+  pdl_wait();  // the weights above are never written; the activations come from the preceding kernel
 
   // the MB activation rows of this pass, once per CTA.  Word 16 jg + 8 h + l of a super-block (group jg, low / high
   // half h, lane l) goes to word 32 (jg / 2) + 4 l + 2 (jg % 2) + h: lane l then reads words 4l..4l+3 of two pieces.
@@ -1027,8 +1005,8 @@ static int32_t q4k_ksplit_launch(rmi_ctx* ctx, const rmi_weight* w, size_t mb, c
     return RMI_ERR_CUDA;
   }
   const dim3 grid((unsigned)((row_end - row_begin + 3) / 4), (unsigned)groups);
-  cudaError_t le = rmi_launch(ctx, kern, grid, dim3(32 * Q4S_WARPS), smem, w->d_raw, nb, w->n_rows, d8, qs, bsums, out, row_begin,
-                              row_end, ctx->d_status);
+  cudaError_t le = rmi_launch_after(ctx, kern, grid, dim3(32 * Q4S_WARPS), smem, w->d_raw, nb, w->n_rows, d8, qs, bsums, out,
+                                    row_begin, row_end, ctx->d_status);
   if (le != cudaSuccess) {
     rmi_set_error("launch of q4k_q8k_ksplit failed: %s", cudaGetErrorString(le));
     return RMI_ERR_CUDA;
@@ -1053,8 +1031,12 @@ static int32_t q4k_stream_launch(rmi_ctx* ctx, const rmi_weight* w, size_t mb, c
   if (grid > n_tiles) grid = n_tiles;
   const size_t tiles_per_cta = (n_tiles + grid - 1) / grid;
   grid = (n_tiles + tiles_per_cta - 1) / tiles_per_cta;   // every CTA walks the same number of tiles
-  kern<<<dim3((unsigned)grid, (unsigned)groups), 32 * Q4S_WARPS, smem, ctx->stream>>>(w->d_raw, nb, w->n_rows, d8, qs, bsums, out,
-                                                                                       row_begin, row_end, n_tiles, ctx->d_status);
+  const cudaError_t le = rmi_launch_after(ctx, kern, dim3((unsigned)grid, (unsigned)groups), dim3(32 * Q4S_WARPS), smem, w->d_raw, nb,
+                                          w->n_rows, d8, qs, bsums, out, row_begin, row_end, n_tiles, ctx->d_status);
+  if (le != cudaSuccess) {
+    rmi_set_error("launch of q4k_q8k_stream failed: %s", cudaGetErrorString(le));
+    return RMI_ERR_CUDA;
+  }
   return rmi_post_launch(ctx, "q4k_q8k_stream");
 }
 
