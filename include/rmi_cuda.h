@@ -90,10 +90,9 @@ int32_t rmi_sync(rmi_ctx* ctx);
  * norm/quantize, attention, SiLU, the Q8_K quantizer and the Q4_K x Q8_K kernels) are launched with programmatic
  * stream serialization: a kernel may start while its predecessor in the stream drains, sets up its barriers and
  * tensor memory, fetches what no earlier kernel writes (its weights), and waits (griddepcontrol.wait) before it
- * touches anything else.  Results are unchanged; chains of dependent kernels run closer together (the M=512 FFN
- * step: 57.7 -> 51.7 us).  Off by default, because a weight uploaded or re-laid-out on the same stream without a
- * synchronisation in between could be fetched before it is complete; the decode session turns it on for its own
- * captured step.  The reference's counterpart is the absence of
+ * touches anything else.  Results are unchanged; chains of dependent kernels run closer together.  On by default:
+ * uploads and re-layouts synchronise before they return, so no weight is fetched before it is complete.  The reference's
+ * counterpart is the absence of
  * a launch gap between operators inside one thread-pool dispatch (src/core/thread_pool.rs:119-161). */
 int32_t rmi_set_dependent_launch(rmi_ctx* ctx, int32_t on);
 /* sm count, L2 bytes, total device memory */

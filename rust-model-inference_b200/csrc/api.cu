@@ -220,7 +220,7 @@ extern "C" int32_t rmi_init(int32_t device, rmi_ctx** out) {
   c->wait_limit_ns = 2000000000ull;
   c->launches = 0;
   c->prof_on = false;
-  c->pdl = false;
+  c->pdl = true;
   c->fanout = out_fanout{};
   c->pipe_ready = false;
   c->pin_in = c->pin_out = c->pin_in_dev = nullptr;
@@ -584,6 +584,11 @@ int32_t ensure_umma_layout(rmi_ctx* ctx, const rmi_weight* cw, bool gate_up_inte
   if (st == RMI_OK && cudaMemsetAsync(s, 0, sb, ctx->stream) != cudaSuccess) st = RMI_ERR_CUDA;
   if (st == RMI_OK)
     st = launch_q8_build_umma(ctx, w->d_tile16, q, s, w->n_rows, blocks, gate_up_interleaved ? w->n_rows_a : 0);
+  // complete before any kernel of a dependent launch may fetch it ahead of its wait
+  if (st == RMI_OK && cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+    rmi_set_error("weight re-layout failed: %s", cudaGetErrorString(cudaGetLastError()));
+    st = RMI_ERR_CUDA;
+  }
   if (st != RMI_OK) {
     cudaFree(q);
     if (s) cudaFree(s);
@@ -692,9 +697,10 @@ extern "C" int32_t rmi_matmul_q8_0_prequantized(rmi_ctx* ctx, const rmi_weight* 
 
 // dout: [m][out_stride] f32, the weight's rows land in columns [0, n_rows); out_stride 0 = n_rows
 int32_t matmul_q8_0_device(rmi_ctx* ctx, const rmi_weight* w, const float* dx, size_t m, float* dout,
-                           size_t out_stride) {
+                           size_t out_stride, bool read_once) {
   const size_t blocks = w->n_in / 32;
   if (out_stride == 0) out_stride = w->n_rows;
+  if (!read_once && q8_gemv_quant_eligible(ctx, w, dx, m)) return launch_q8_gemv_quant(ctx, w, dx, m, dout, out_stride);
   if (matmul_on_tensor_cores(ctx, m)) {
     RMI_TRY(ensure_umma_layout(ctx, w));
     const size_t m_tiles = (m + 127) / 128, n_slabs = (w->n_in + 127) / 128;
@@ -766,9 +772,9 @@ extern "C" int32_t rmi_matmul_q8_0(rmi_ctx* ctx, const rmi_weight* w, const floa
   RMI_REQUIRE(x && output, RMI_ERR_BAD_HANDLE, "rmi_matmul_q8_0: null buffer");
   std::lock_guard<std::mutex> lock(ctx->mu);
   float *dx, *dout;
-  RMI_TRY(host_in(ctx, x, m * w->n_in * 4, 5, m > 1, (void**)&dx));  // one row may be quantized by every CTA
+  RMI_TRY(host_in(ctx, x, m * w->n_in * 4, 5, true, (void**)&dx));
   RMI_TRY(rmi_scratch(ctx, 6, m * w->n_rows * 4, (void**)&dout));
-  RMI_TRY(matmul_q8_0_device(ctx, w, dx, m, dout));
+  RMI_TRY(matmul_q8_0_device(ctx, w, dx, m, dout, 0, true));
   RMI_TRY(host_out(ctx, output, dout, 1, m * w->n_rows * 4, 0));
   return matmul_on_tensor_cores(ctx, m) ? rmi_check_dev_status(ctx, "rmi_matmul_q8_0") : RMI_OK;
 }
@@ -854,7 +860,7 @@ extern "C" int32_t rmi_q8_0_block_sums(rmi_ctx* ctx, const rmi_weight* w, const 
 // ---------------------------------------------------------------- fused SwiGLU FFN
 
 int32_t ffn_device(rmi_ctx* ctx, const rmi_weight* wgu, const rmi_weight* wd, const float* dx, size_t m,
-                   float* dout) {
+                   float* dout, bool read_once) {
   const size_t n_embd = wgu->n_in, n_ff = wgu->n_rows / 2;
   RMI_REQUIRE(wgu->n_rows_a * 2 == wgu->n_rows && wgu->n_rows_a > 0, RMI_ERR_BAD_SHAPE,
               "w_gate_up must be rmi_weight_fuse_vstack(gate, up) of equal row counts");
@@ -910,8 +916,12 @@ int32_t ffn_device(rmi_ctx* ctx, const rmi_weight* wgu, const rmi_weight* wd, co
   RMI_TRY(rmi_scratch(ctx, 2, m * 2 * n_ff * 4, (void**)&gu));
   RMI_TRY(rmi_scratch(ctx, 3, m * n_ff, (void**)&q2));
   RMI_TRY(rmi_scratch(ctx, 4, m * b2 * 4, (void**)&sc2));
-  RMI_TRY(launch_q8_quantize(ctx, dx, m, n_embd, q1, sc1, 0));
-  RMI_TRY(launch_q8_gemv(ctx, wgu, q1, sc1, m, gu, 2 * n_ff, 0, 2 * n_ff));
+  if (!read_once && q8_gemv_quant_eligible(ctx, wgu, dx, m)) {
+    RMI_TRY(launch_q8_gemv_quant(ctx, wgu, dx, m, gu, 2 * n_ff));
+  } else {
+    RMI_TRY(launch_q8_quantize(ctx, dx, m, n_embd, q1, sc1, 0));
+    RMI_TRY(launch_q8_gemv(ctx, wgu, q1, sc1, m, gu, 2 * n_ff, 0, 2 * n_ff));
+  }
   RMI_TRY(launch_silu_mul_quantize(ctx, gu, gu + n_ff, 2 * n_ff, m, n_ff, nullptr, q2, sc2));
   return launch_q8_gemv(ctx, wd, q2, sc2, m, dout, n_embd, 0, n_embd);
 }
@@ -937,7 +947,7 @@ extern "C" int32_t rmi_ffn_swiglu_q8_0(rmi_ctx* ctx, const rmi_weight* wgu, cons
   float *dx, *dout;
   RMI_TRY(host_in(ctx, x, m * wgu->n_in * 4, 5, true, (void**)&dx));
   RMI_TRY(rmi_scratch(ctx, 6, m * wd->n_rows * 4, (void**)&dout));
-  RMI_TRY(ffn_device(ctx, wgu, wd, dx, m, dout));
+  RMI_TRY(ffn_device(ctx, wgu, wd, dx, m, dout, true));
   RMI_TRY(host_out(ctx, out, dout, 1, m * wd->n_rows * 4, 0));
   return use_tensor_cores(ctx, m) ? rmi_check_dev_status(ctx, "rmi_ffn_swiglu_q8_0") : RMI_OK;
 }

@@ -9,6 +9,9 @@ int32_t launch_q8_build_umma(rmi_ctx* ctx, const uint8_t* t16, uint8_t* uq, floa
 int32_t launch_q8_quantize(rmi_ctx* ctx, const float* x, size_t m, size_t n, uint8_t* q8, float* scales, int out_mode);
 int32_t launch_q8_gemv(rmi_ctx* ctx, const rmi_weight* w, const uint8_t* xq, const float* xs, size_t m,
                        float* out, size_t out_stride, size_t row_begin, size_t row_end);
+// quantize + GEMV in one kernel for few f32 rows
+bool q8_gemv_quant_eligible(const rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m);
+int32_t launch_q8_gemv_quant(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, float* out, size_t out_stride);
 bool q8_gemv_fused_norm_eligible(const rmi_ctx* ctx, const rmi_weight* w, size_t m);
 // x = x_in (+ add); rms_norm(x, norm_w, eps); quantize; out = W x.  x is also written to x_out (!= x_in).
 int32_t launch_q8_matmul_f32(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, float* out);
@@ -42,10 +45,11 @@ int32_t launch_gemm_tc(rmi_ctx* ctx, const gemm_tc_args& a);
 int32_t ensure_umma_layout(rmi_ctx* ctx, const rmi_weight* w, bool gate_up_interleaved = false);
 
 // api.cu: quantize + matmul / fused FFN on device buffers (caller holds ctx->mu); dout [m][out_stride],
-// out_stride 0 = n_rows.  Uses the context's scratch slots 0..4.
+// out_stride 0 = n_rows.  Uses the context's scratch slots 0..4.  read_once: dx is mapped host memory, one kernel reads it.
 int32_t matmul_q8_0_device(rmi_ctx* ctx, const rmi_weight* w, const float* dx, size_t m, float* dout,
-                           size_t out_stride = 0);
-int32_t ffn_device(rmi_ctx* ctx, const rmi_weight* wgu, const rmi_weight* wd, const float* dx, size_t m, float* dout);
+                           size_t out_stride = 0, bool read_once = false);
+int32_t ffn_device(rmi_ctx* ctx, const rmi_weight* wgu, const rmi_weight* wd, const float* dx, size_t m, float* dout,
+                   bool read_once = false);
 
 // peer.cu: writes `epoch` into slot `rank` of every flag array, then waits (at most ctx->wait_limit_ns) until
 // all `world` slots of flags[rank] reached it; on `stream`

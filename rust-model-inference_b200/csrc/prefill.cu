@@ -25,6 +25,8 @@ namespace {
 // x[r][:] = f16(d) * q of row prompts[b][p]; r = b_local * P + p
 __global__ void embed_rows_kernel(const uint8_t* __restrict__ emb, size_t blocks, const uint32_t* __restrict__ prompts,
                                   size_t n_prompt, size_t P, size_t b0, float* __restrict__ x, uint32_t vocab) {
+  pdl_wait();
+  pdl_launch_dependents();
   const size_t r = blockIdx.x, b = b0 + r / P, p = r % P;
   uint32_t tok = prompts[b * n_prompt + p];
   if (tok >= vocab) tok = 0;  // rejected on the host before the first launch
@@ -40,6 +42,8 @@ __global__ void embed_rows_kernel(const uint8_t* __restrict__ emb, size_t blocks
 // x += add (optional); out = rms_norm(x) * weight.  One CTA of 256 threads per row.
 __global__ void rmsnorm_rows_kernel(float* __restrict__ x, const float* __restrict__ add, const float* __restrict__ weight,
                                     size_t n, float eps, float* __restrict__ out) {
+  pdl_wait();
+  pdl_launch_dependents();
   __shared__ double s_part[8];
   __shared__ float s_scale;
   const size_t r = blockIdx.x;
@@ -74,6 +78,8 @@ __global__ void qk_norm_rope_kv_rows_kernel(const float* __restrict__ qkv, size_
                                             const float* __restrict__ rope, size_t P, size_t b0,
                                             uint16_t* __restrict__ q16, uint16_t* __restrict__ k_cache,
                                             uint16_t* __restrict__ v_cache, size_t layer, size_t n_layer, size_t capacity) {
+  pdl_wait();
+  pdl_launch_dependents();
   const size_t r = blockIdx.x, head = blockIdx.y, b = b0 + r / P, p = r % P;
   const int lane = threadIdx.x;
   const size_t nq = n_head * hd, nk = n_head_kv * hd;
@@ -102,6 +108,8 @@ __global__ void __launch_bounds__(256)
     attention_prefill_kernel(const uint16_t* __restrict__ q16, const uint16_t* __restrict__ k_cache,
                              const uint16_t* __restrict__ v_cache, size_t n_head, size_t n_head_kv, size_t layer,
                              size_t n_layer, size_t capacity, size_t P, size_t b0, int QT, float* __restrict__ attn_out) {
+  pdl_wait();
+  pdl_launch_dependents();
   extern __shared__ __align__(16) uint8_t smem[];
   const size_t kvh = blockIdx.y, bl = blockIdx.z, b = b0 + bl;
   const int t_first = (int)blockIdx.x * QT;
@@ -225,7 +233,11 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-__global__ void set_step_kernel(int* d_step, int value) { *d_step = value; }
+__global__ void set_step_kernel(int* d_step, int value) {
+  pdl_wait();
+  pdl_launch_dependents();
+  *d_step = value;
+}
 
 size_t prefill_attention_smem(int QT, int group, size_t T, size_t hd) {
   const size_t cs = (T + 7) & ~(size_t)7, rows = (size_t)QT * group;
@@ -254,24 +266,21 @@ bool prefill_supported(const rmi_ctx* ctx, const decode_dims& d, size_t P) {
 
 int32_t launch_embed_rows(rmi_ctx* ctx, const rmi_weight* emb, const uint32_t* prompts, size_t n_prompt, size_t P, size_t b0,
                           size_t rows, float* x) {
-  embed_rows_kernel<<<(unsigned)rows, 256, 0, ctx->stream>>>(emb->d_tile16, emb->n_in / 32, prompts, n_prompt, P, b0, x,
-                                                           (uint32_t)emb->n_rows);
-  return rmi_post_launch(ctx, "embed_rows");
+  return rmi_run(ctx, "embed_rows", embed_rows_kernel, dim3((unsigned)rows), dim3(256), 0, emb->d_tile16, emb->n_in / 32, prompts,
+                 n_prompt, P, b0, x, (uint32_t)emb->n_rows);
 }
 
 int32_t launch_rmsnorm_rows(rmi_ctx* ctx, float* x, const float* add, const float* weight, size_t n, float eps, float* out,
                             size_t rows) {
-  rmsnorm_rows_kernel<<<(unsigned)rows, 256, 0, ctx->stream>>>(x, add, weight, n, eps, out);
-  return rmi_post_launch(ctx, "rmsnorm_rows");
+  return rmi_run(ctx, "rmsnorm_rows", rmsnorm_rows_kernel, dim3((unsigned)rows), dim3(256), 0, x, add, weight, n, eps, out);
 }
 
 int32_t launch_qk_norm_rope_kv_rows(rmi_ctx* ctx, const decode_dims& d, const float* qkv, const float* q_norm,
                                     const float* k_norm, const float* rope, size_t P, size_t b0, size_t rows, uint16_t* q16,
                                     uint16_t* k_cache, uint16_t* v_cache, size_t layer) {
   dim3 grid((unsigned)rows, (unsigned)(d.n_head + 2 * d.n_head_kv));
-  qk_norm_rope_kv_rows_kernel<<<grid, 32, 0, ctx->stream>>>(qkv, d.n_head, d.n_head_kv, d.hd, q_norm, k_norm, d.eps, rope, P,
-                                                            b0, q16, k_cache, v_cache, layer, d.n_layer, d.capacity);
-  return rmi_post_launch(ctx, "qk_norm_rope_kv_rows");
+  return rmi_run(ctx, "qk_norm_rope_kv_rows", qk_norm_rope_kv_rows_kernel, grid, dim3(32), 0, qkv, d.n_head, d.n_head_kv, d.hd, q_norm,
+                 k_norm, d.eps, rope, P, b0, q16, k_cache, v_cache, layer, d.n_layer, d.capacity);
 }
 
 int32_t launch_attention_prefill(rmi_ctx* ctx, const decode_dims& d, const uint16_t* q16, const uint16_t* k_cache,
@@ -289,12 +298,10 @@ int32_t launch_attention_prefill(rmi_ctx* ctx, const decode_dims& d, const uint1
     return RMI_ERR_UNSUPPORTED;
   }
   dim3 grid((unsigned)((P + qt - 1) / qt), (unsigned)d.n_head_kv, (unsigned)n_seq);
-  kern<<<grid, 256, smem, ctx->stream>>>(q16, k_cache, v_cache, d.n_head, d.n_head_kv, layer, d.n_layer, d.capacity, P, b0, qt,
-                                         attn_out);
-  return rmi_post_launch(ctx, "attention_prefill");
+  return rmi_run(ctx, "attention_prefill", kern, grid, dim3(256), smem, q16, k_cache, v_cache, d.n_head, d.n_head_kv, layer, d.n_layer,
+                 d.capacity, P, b0, qt, attn_out);
 }
 
 int32_t launch_set_step(rmi_ctx* ctx, int* d_step, int value) {
-  set_step_kernel<<<1, 1, 0, ctx->stream>>>(d_step, value);
-  return rmi_post_launch(ctx, "set_step");
+  return rmi_run(ctx, "set_step", set_step_kernel, dim3(1), dim3(1), 0, d_step, value);
 }

@@ -140,7 +140,7 @@ static int32_t q4_0_launch(rmi_ctx* ctx, const rmi_weight* w, const uint8_t* xq,
     return RMI_ERR_CUDA;
   }
   const dim3 grid((unsigned)((row_end - row_begin + Q40_ROWS - 1) / Q40_ROWS), (unsigned)groups);
-  const cudaError_t le = rmi_launch_after(ctx, kern, grid, dim3(Q40_THREADS), smem, w->d_raw, blocks, w->n_rows, xq, xs, out,
+  const cudaError_t le = rmi_launch(ctx, kern, grid, dim3(Q40_THREADS), smem, w->d_raw, blocks, w->n_rows, xq, xs, out,
                                           row_begin, row_end);
   if (le != cudaSuccess) {
     rmi_set_error("launch of q4_0_matmul failed: %s", cudaGetErrorString(le));

@@ -100,10 +100,6 @@ __device__ __forceinline__ void scale_min_w(uint32_t w1, uint32_t w2, uint32_t w
 // Super-blocks of a row are fetched Q4K_U at a time: lane h loads the 16-byte header of super-block i0+h (one
 // load instead of a dozen dependent byte loads) and every lane its 4 quant bytes of each of the Q4K_U blocks,
 // all issued before the first use; the header fields reach the lanes by shuffle (Q4K_U = q4k_batch<MP>::U).
-#ifndef RMI_Q4K_ROWS8
-#define RMI_Q4K_ROWS8 2
-#endif
-
 template <int MP>
 struct q4k_batch {
   static constexpr int U = MP >= 4 ? 8 : 16;  // fewer blocks in flight when the accumulators need the registers
@@ -117,6 +113,8 @@ __global__ void q4k_q8k_matmul_kernel(const uint8_t* __restrict__ w, size_t nb, 
                                       const int16_t* __restrict__ bs, float* __restrict__ out, size_t row_begin,
                                       size_t row_end) {
   constexpr int Q4K_U = q4k_batch<MP>::U;
+  pdl_wait();
+  pdl_launch_dependents();
   const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
   const int lane = threadIdx.x & 31;
   const size_t row = row_begin + warp;
@@ -264,6 +262,8 @@ __global__ void __launch_bounds__(256)
   __shared__ int s_xs[2][Q4T_TM][8];                       // pairwise bsum sums (i16 wrap): [tt][0], [tt][1]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int L = lane & 7, tm = lane >> 3, tn = warp;       // 4 activation-row tiles per warp share the weight tile
+  pdl_wait();
+  pdl_launch_dependents();
   const size_t n0 = row_begin + (size_t)blockIdx.x * Q4T_TN, m0 = (size_t)blockIdx.y * Q4T_TM;
 
   auto load_stage = [&](int st, size_t i) {
@@ -735,6 +735,8 @@ __global__ void q4k_dequant_matmul_kernel(const uint8_t* __restrict__ w, size_t 
   const size_t row0 = (((size_t)blockIdx.x * blockDim.x + threadIdx.x) / 32) * R;
   const int lane = threadIdx.x & 31;
   if (row0 >= n_rows) return;
+  pdl_wait();
+  pdl_launch_dependents();
   const int j = lane / 8, L = lane % 8;
   const size_t K = nb * 256;
   float acc[R][MP];
@@ -837,6 +839,8 @@ __global__ void __launch_bounds__(256 * Q4G_KGROUPS)
     q4k_dequant_gemm_kernel(const uint8_t* __restrict__ w, size_t nb, size_t n_rows, const float* __restrict__ x,
                             size_t m_rows, float* __restrict__ out) {
   extern __shared__ __align__(16) uint8_t q4g_smem[];
+  pdl_wait();
+  pdl_launch_dependents();
   const int kg = threadIdx.x >> 8, tid = threadIdx.x & 255;
   uint8_t* gsm = q4g_smem + (size_t)kg * Q4G_GROUP_SMEM;
   float (*Ws)[Q4G_BK][Q4G_BN + Q4G_PAD] = reinterpret_cast<float (*)[Q4G_BK][Q4G_BN + Q4G_PAD]>(gsm);
@@ -992,7 +996,8 @@ static void q4k_q8k_launch(rmi_ctx* ctx, const rmi_weight* w, const float* d8, c
   const size_t rows = row_end - row_begin, nb = w->n_in / 256;
   dim3 grid((unsigned)((rows + 3) / 4), (unsigned)groups);
   // only the scalar order runs here; the AVX2 order has the kernels above
-  q4k_q8k_matmul_kernel<RMI_SEM_SCALAR, MP><<<grid, 128, 0, ctx->stream>>>(w->d_raw, nb, w->n_rows, d8, qs, bsums, out, row_begin, row_end);
+  (void)rmi_launch(ctx, q4k_q8k_matmul_kernel<RMI_SEM_SCALAR, MP>, grid, dim3(128), 0, w->d_raw, nb, w->n_rows, d8, qs, bsums, out,
+                   row_begin, row_end);
 }
 
 // One launch of the split-K kernel over `groups` groups of mb (1 or 2) activation rows.
@@ -1005,7 +1010,7 @@ static int32_t q4k_ksplit_launch(rmi_ctx* ctx, const rmi_weight* w, size_t mb, c
     return RMI_ERR_CUDA;
   }
   const dim3 grid((unsigned)((row_end - row_begin + 3) / 4), (unsigned)groups);
-  cudaError_t le = rmi_launch_after(ctx, kern, grid, dim3(32 * Q4S_WARPS), smem, w->d_raw, nb, w->n_rows, d8, qs, bsums, out,
+  cudaError_t le = rmi_launch(ctx, kern, grid, dim3(32 * Q4S_WARPS), smem, w->d_raw, nb, w->n_rows, d8, qs, bsums, out,
                                     row_begin, row_end, ctx->d_status);
   if (le != cudaSuccess) {
     rmi_set_error("launch of q4k_q8k_ksplit failed: %s", cudaGetErrorString(le));
@@ -1031,7 +1036,7 @@ static int32_t q4k_stream_launch(rmi_ctx* ctx, const rmi_weight* w, size_t mb, c
   if (grid > n_tiles) grid = n_tiles;
   const size_t tiles_per_cta = (n_tiles + grid - 1) / grid;
   grid = (n_tiles + tiles_per_cta - 1) / tiles_per_cta;   // every CTA walks the same number of tiles
-  const cudaError_t le = rmi_launch_after(ctx, kern, dim3((unsigned)grid, (unsigned)groups), dim3(32 * Q4S_WARPS), smem, w->d_raw, nb,
+  const cudaError_t le = rmi_launch(ctx, kern, dim3((unsigned)grid, (unsigned)groups), dim3(32 * Q4S_WARPS), smem, w->d_raw, nb,
                                           w->n_rows, d8, qs, bsums, out, row_begin, row_end, n_tiles, ctx->d_status);
   if (le != cudaSuccess) {
     rmi_set_error("launch of q4k_q8k_stream failed: %s", cudaGetErrorString(le));
@@ -1047,8 +1052,8 @@ int32_t launch_q4k_q8k_matmul(rmi_ctx* ctx, const rmi_weight* w, const float* d8
   if (m >= 32 && ctx->sem != RMI_SEM_SCALAR) {
     // many rows: tiled kernel, every weight super-block is fetched once per 16 activation rows
     dim3 grid((unsigned)((row_end - row_begin + Q4T_TN - 1) / Q4T_TN), (unsigned)((m + Q4T_TM - 1) / Q4T_TM));
-    q4k_q8k_tiled_kernel<<<grid, 256, 0, ctx->stream>>>(w->d_raw, nb, w->n_rows, d8, qs, bsums, m, out, row_begin, row_end);
-    return rmi_post_launch(ctx, "q4k_q8k_tiled");
+    return rmi_run(ctx, "q4k_q8k_tiled", q4k_q8k_tiled_kernel, grid, dim3(256), 0, w->d_raw, nb, w->n_rows, d8, qs, bsums, m, out,
+                   row_begin, row_end);
   }
   if (ctx->sem != RMI_SEM_SCALAR) {
     // few rows: groups of 8 / 4 activation rows through the streaming kernel (16-row tiles, whole rows per warp),
@@ -1095,29 +1100,19 @@ int32_t launch_q4k_dequant_matmul(rmi_ctx* ctx, const rmi_weight* w, const float
       rmi_set_error("cudaFuncSetAttribute(%zu B shared) failed", smem);
       return RMI_ERR_CUDA;
     }
-    q4k_dequant_gemm_kernel<<<g2, 256 * Q4G_KGROUPS, smem, ctx->stream>>>(w->d_raw, nb, w->n_rows, x, m, out);
-    return rmi_post_launch(ctx, "q4k_dequant_gemm");
+    return rmi_run(ctx, "q4k_dequant_gemm", q4k_dequant_gemm_kernel, g2, dim3(256 * Q4G_KGROUPS), smem, w->d_raw, nb, w->n_rows, x, m, out);
   }
   size_t t = 0;
   while (t < m) {
     const size_t left = m - t;
     const float* xp = x + t * w->n_in;
     float* op = out + t * w->n_rows;
-    if (left >= 8) {
-      constexpr int R = RMI_Q4K_ROWS8;
-      q4k_dequant_matmul_kernel<8, R><<<(unsigned)((w->n_rows + 4 * R - 1) / (4 * R)), 128, 0, ctx->stream>>>(w->d_raw, nb, w->n_rows, xp, op);
-      t += 8;
-    } else if (left >= 4) {
-      q4k_dequant_matmul_kernel<4, 2><<<(unsigned)((w->n_rows + 7) / 8), 128, 0, ctx->stream>>>(w->d_raw, nb, w->n_rows, xp, op);
-      t += 4;
-    } else if (left >= 2) {
-      q4k_dequant_matmul_kernel<2, 1><<<(unsigned)((w->n_rows + 3) / 4), 128, 0, ctx->stream>>>(w->d_raw, nb, w->n_rows, xp, op);
-      t += 2;
-    } else {
-      q4k_dequant_matmul_kernel<1, 1><<<(unsigned)((w->n_rows + 3) / 4), 128, 0, ctx->stream>>>(w->d_raw, nb, w->n_rows, xp, op);
-      t += 1;
-    }
-    RMI_TRY(rmi_post_launch(ctx, "q4k_dequant_matmul"));
+    const size_t mp = left >= 8 ? 8 : (left >= 4 ? 4 : (left >= 2 ? 2 : 1)), rows_per_cta = mp >= 4 ? 8 : 4;   // 4 warps of 2 or 1 rows
+    auto kern = mp == 8 ? q4k_dequant_matmul_kernel<8, 2>
+                        : (mp == 4 ? q4k_dequant_matmul_kernel<4, 2> : (mp == 2 ? q4k_dequant_matmul_kernel<2, 1> : q4k_dequant_matmul_kernel<1, 1>));
+    RMI_TRY(rmi_run(ctx, "q4k_dequant_matmul", kern, dim3((unsigned)((w->n_rows + rows_per_cta - 1) / rows_per_cta)), dim3(128), 0,
+                    w->d_raw, nb, w->n_rows, xp, op));
+    t += mp;
   }
   return RMI_OK;
 }

@@ -336,7 +336,7 @@ int32_t q6k_stream_launch(rmi_ctx* ctx, const rmi_weight* w, const float* d8, co
   if (grid > n_tiles) grid = n_tiles;
   const size_t tiles_per_cta = (n_tiles + grid - 1) / grid;
   grid = (n_tiles + tiles_per_cta - 1) / tiles_per_cta;   // every CTA walks the same number of tiles
-  const cudaError_t le = rmi_launch_after(ctx, kern, dim3((unsigned)grid, (unsigned)groups), dim3(32 * Q6S_WARPS), smem, w->d_raw,
+  const cudaError_t le = rmi_launch(ctx, kern, dim3((unsigned)grid, (unsigned)groups), dim3(32 * Q6S_WARPS), smem, w->d_raw,
                                           nb, w->n_rows, d8, qs, bsums, out, row_begin, row_end, n_tiles, ctx->d_status);
   if (le != cudaSuccess) {
     rmi_set_error("launch of q6k_q8k_stream failed: %s", cudaGetErrorString(le));

@@ -75,38 +75,49 @@ __global__ void q8_build_umma_kernel(const uint8_t* __restrict__ t16, uint8_t* _
 
 // ---------------------------------------------------------------- activation quantizer
 
-// One warp per 32-block.  out_mode 0: q8 row-major [m][n], scales [m][n/32].
+// Eight threads per 32-block, thread L the four values 4L..4L+3 (one 16-byte load, one 4-byte store).
+// out_mode 0: q8 row-major [m][n], scales [m][n/32].
 // out_mode 1: q8 in tcgen05 A-operand images ([tile128][slab][16 KiB]) and scales
 // [tile128][block][128]; rows m..pad are written as zeros by the caller's memset.
+// aligned: x on a 16-byte boundary and q8 on a 4-byte boundary; otherwise single elements are moved.
 template <int SEM>
-__global__ void q8_quantize_kernel(const float* __restrict__ x, size_t m, size_t n,
-                                   uint8_t* __restrict__ q8, float* __restrict__ scales,
-                                   int out_mode) {
+__global__ void __launch_bounds__(256)
+    q8_quantize_kernel(const float* __restrict__ x, size_t n_words, size_t blocks, uint8_t* __restrict__ q8,
+                       float* __restrict__ scales, int out_mode, int aligned) {
   pdl_wait();               // x may come from the preceding kernel of a dependent launch
   pdl_launch_dependents();
-  size_t blocks = n / 32;
-  size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
-  int lane = threadIdx.x & 31;
-  if (warp >= m * blocks) return;
-  size_t row = warp / blocks, b = warp % blocks;
-  float v = x[row * n + b * 32 + lane];
-  float a = fabsf(v);
+  const size_t word = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool ok = word < n_words;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (ok) {
+    if (aligned) v = __ldg(reinterpret_cast<const float4*>(x) + word);
+    else v = make_float4(__ldg(x + 4 * word), __ldg(x + 4 * word + 1), __ldg(x + 4 * word + 2), __ldg(x + 4 * word + 3));
+  }
+  float a = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
+  for (int o = 4; o > 0; o >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
+  if (!ok) return;
   float d, inv;
   q8_scale_pair<SEM>(a, &d, &inv);
-  int q = q8_quant_value<SEM>(v, inv);
-  float sc = f16_round_trip(d);
+  const int q[4] = {q8_quant_value<SEM>(v.x, inv), q8_quant_value<SEM>(v.y, inv), q8_quant_value<SEM>(v.z, inv),
+                    q8_quant_value<SEM>(v.w, inv)};
+  const uint32_t packed = (uint32_t)(q[0] & 0xff) | (uint32_t)(q[1] & 0xff) << 8 | (uint32_t)(q[2] & 0xff) << 16 | (uint32_t)(q[3] & 0xff) << 24;
+  const size_t blk = word / 8, row = blk / blocks, b = blk - row * blocks;
+  const int L = (int)(word & 7);
+  const float sc = f16_round_trip(d);
   if (out_mode == 0) {
-    q8[row * n + b * 32 + lane] = (uint8_t)(int8_t)q;
-    if (lane == 0) scales[row * blocks + b] = sc;
+    if (aligned) {
+      reinterpret_cast<uint32_t*>(q8)[word] = packed;
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; k++) q8[4 * word + k] = (uint8_t)(packed >> (8 * k));
+    }
+    if (L == 0) scales[blk] = sc;
   } else {
-    size_t n_slabs = (n + 127) / 128;
-    size_t tile = row / 128, r = row % 128, k = b * 32 + lane;
-    size_t slab = k / 128, c = (k % 128) / 16, byte = k % 16;
-    q8[(tile * n_slabs + slab) * 16384 + (r / 8) * 1024 + c * 128 + (r % 8) * 16 + byte] =
-        (uint8_t)(int8_t)q;
-    if (lane == 0) scales[(tile * blocks + b) * 128 + r] = sc;
+    const size_t n_slabs = (blocks + 3) / 4, tile = row / 128, r = row % 128, k = b * 32 + 4 * L;
+    const size_t slab = k / 128, c = (k % 128) / 16, byte = k % 16;
+    *reinterpret_cast<uint32_t*>(q8 + (tile * n_slabs + slab) * 16384 + (r / 8) * 1024 + c * 128 + (r % 8) * 16 + byte) = packed;
+    if (L == 0) scales[(tile * blocks + b) * 128 + r] = sc;
   }
 }
 
@@ -431,10 +442,13 @@ __global__ void __launch_bounds__(256)
 // the tile costs one memory round trip; thread (row r, lane l) then runs the reference's
 // per-lane chain over the blocks out of shared memory.
 //
-// FUSED: the activations are not read pre-quantized; every CTA derives them itself while its
+// STAGED_NORM: the activations are not read pre-quantized; every CTA derives them itself while its
 // weight copy is in flight: x = x_in (+ add), rms_norm(x, norm_w) (src/ops/norm.rs:3-11), Q8_0
 // quantization.  The updated residual stream is written to x_out by the CTAs of tile 0 only
 // (x_out must not alias x_in: other CTAs are still reading it).
+// STAGED_QUANT: the same with the quantization alone, for a matmul of few f32 rows: one launch instead of two, and the
+// quantizer's time disappears behind the weight copy (3072 x 1024, one row: 8.2 -> 3.5 us per call).
+enum { STAGED_PLAIN = 0, STAGED_NORM = 1, STAGED_QUANT = 2 };
 struct gemv_norm_args {
   const float* x_in;
   const float* add;     // may be null
@@ -443,12 +457,13 @@ struct gemv_norm_args {
   float eps;
 };
 
-template <int SEM, int MP, bool FUSED>
+template <int SEM, int MP, int MODE>
 __global__ void __launch_bounds__(128)
     q8_gemv_staged_kernel(const uint8_t* __restrict__ w, size_t blocks, const uint8_t* __restrict__ xq,
                           const float* __restrict__ xs, float* __restrict__ out, size_t out_stride, size_t row_begin,
                           size_t row_end, size_t first_tile, rmi_dev_status* status, gemv_norm_args na,
                           const out_fanout fo) {
+  constexpr bool FUSED = MODE == STAGED_NORM;
   extern __shared__ __align__(128) uint8_t smem[];
   const size_t K = blocks * 32;
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
@@ -456,7 +471,7 @@ __global__ void __launch_bounds__(128)
   int8_t* xq_s = reinterpret_cast<int8_t*>(wt + blocks * Q8_REC_BYTES);  // [MP][K]
   float* xs_s = reinterpret_cast<float*>(xq_s + MP * K);      // [MP][blocks]
   float* xf = xs_s + MP * blocks;                             // [MP][K], FUSED only
-  if (!FUSED) {
+  if (MODE == STAGED_PLAIN) {
     xq += (size_t)blockIdx.y * MP * K;
     xs += (size_t)blockIdx.y * MP * blocks;
   }
@@ -491,7 +506,31 @@ __global__ void __launch_bounds__(128)
   }
   pdl_wait();  // the weight copy above is in flight; everything below depends on the previous kernel
   pdl_launch_dependents();
-  if (!FUSED) {
+  if constexpr (MODE == STAGED_QUANT) {
+    // eight threads per 32-block, four values each; four blocks per thread in flight
+    const int n_words = (int)(MP * K / 4), L = threadIdx.x & 7;
+    const float4* xv = reinterpret_cast<const float4*>(na.x_in + (size_t)blockIdx.y * MP * K);
+    for (int w0 = threadIdx.x; w0 < n_words; w0 += 4 * 128) {
+      float4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) v[u] = w0 + u * 128 < n_words ? __ldg(xv + w0 + u * 128) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        float a = fmaxf(fmaxf(fabsf(v[u].x), fabsf(v[u].y)), fmaxf(fabsf(v[u].z), fabsf(v[u].w)));
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) a = fmaxf(a, __shfl_xor_sync(__activemask(), a, o));   // whole groups of eight are active
+        const int word = w0 + u * 128;
+        if (word < n_words) {
+          float d, inv;
+          q8_scale_pair<SEM>(a, &d, &inv);
+          const uint32_t q0 = (uint32_t)q8_quant_value<SEM>(v[u].x, inv) & 0xffu, q1 = (uint32_t)q8_quant_value<SEM>(v[u].y, inv) & 0xffu;
+          const uint32_t q2 = (uint32_t)q8_quant_value<SEM>(v[u].z, inv) & 0xffu, q3 = (uint32_t)q8_quant_value<SEM>(v[u].w, inv) & 0xffu;
+          reinterpret_cast<uint32_t*>(xq_s)[word] = q0 | q1 << 8 | q2 << 16 | q3 << 24;
+          if (L == 0) xs_s[word >> 3] = f16_round_trip(d);
+        }
+      }
+    }
+  } else if constexpr (!FUSED) {
     // activations, in parallel with the weight copy: asynchronous copies straight into shared memory, all of a
     // thread's pieces in flight at once (a load / store loop through registers waits for each batch in turn)
     for (size_t i = threadIdx.x; i < MP * K / 16; i += blockDim.x)
@@ -861,6 +900,8 @@ template <int SEM>
 __global__ void __launch_bounds__(256)
     q8_matmul_f32_kernel(const uint8_t* __restrict__ w, size_t blocks, size_t n_rows, const float* __restrict__ x,
                          float* __restrict__ out) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int rit = threadIdx.x >> 4, c = threadIdx.x & 15;
   const size_t tile = blockIdx.x, row = tile * 16 + rit, K = blocks * 32;
   const float* xr = x + (size_t)blockIdx.y * K;
@@ -925,17 +966,13 @@ int32_t launch_q8_build_umma(rmi_ctx* ctx, const uint8_t* t16, uint8_t* uq, floa
 
 int32_t launch_q8_quantize(rmi_ctx* ctx, const float* x, size_t m, size_t n, uint8_t* q8, float* scales,
                            int out_mode) {
-  size_t warps = m * (n / 32);
-  if (warps == 0) return RMI_OK;
-  unsigned grid = (unsigned)((warps + 7) / 8);
+  const size_t words = m * (n / 4);
+  if (words == 0) return RMI_OK;
   auto kern = ctx->sem == RMI_SEM_AVX2 ? q8_quantize_kernel<RMI_SEM_AVX2>
                                        : (ctx->sem == RMI_SEM_NEON ? q8_quantize_kernel<RMI_SEM_NEON> : q8_quantize_kernel<RMI_SEM_SCALAR>);
-  const cudaError_t le = rmi_launch(ctx, kern, dim3(grid), dim3(256), 0, x, m, n, q8, scales, out_mode);
-  if (le != cudaSuccess) {
-    rmi_set_error("launch of q8_quantize failed: %s", cudaGetErrorString(le));
-    return RMI_ERR_CUDA;
-  }
-  return rmi_post_launch(ctx, "q8_quantize");
+  const int aligned = ((uintptr_t)x & 15) == 0 && ((uintptr_t)q8 & 3) == 0;
+  return rmi_run(ctx, "q8_quantize", kern, dim3((unsigned)((words + 255) / 256)), dim3(256), 0, x, words, n / 32, q8, scales, out_mode,
+                 aligned);
 }
 
 template <int SEM, int LB, int MP>
@@ -991,7 +1028,7 @@ static int32_t gemv_dispatch_lb(rmi_ctx* ctx, const rmi_weight* w, const uint8_t
     // wider passes only while two CTAs fit on an SM (an 8192-column tile with eight activation rows takes a whole SM
     // and ran slower than the register-staged kernel: 92 against 55 us for 4096 x 8192 at M = 16)
     if (t1 * n_groups <= (size_t)ctx->sm_count * 6 && smem <= ctx->smem_optin - 1024 && (MP <= 2 || smem <= 100 * 1024)) {
-      auto kern = q8_gemv_staged_kernel<SEM, MP, false>;
+      auto kern = q8_gemv_staged_kernel<SEM, MP, STAGED_PLAIN>;
       if (smem > 48 * 1024 &&
           cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
         rmi_set_error("cudaFuncSetAttribute(%zu B shared) failed", smem);
@@ -1089,10 +1126,48 @@ bool q8_gemv_fused_norm_eligible(const rmi_ctx* ctx, const rmi_weight* w, size_t
   return (m == 1 || m == 2) && w->n_tiles16 <= (size_t)ctx->sm_count * 6 && gemv_fused_smem(w, m) <= ctx->smem_optin - 1024;
 }
 
+// ---- quantize + staged GEMV in one kernel ----
+// Shapes of the staged kernel (at most six CTAs per SM, and at least two on an SM) whose rows are few enough that
+// quantizing them in every CTA stays below the latency of its weight copy.
+bool q8_gemv_quant_eligible(const rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m) {
+  const size_t blocks = w->n_in / 32, smem = 128 + blocks * Q8_REC_BYTES + m * (w->n_in + blocks * 4);
+  return (m == 1 || m == 2 || m == 4) && m * w->n_in <= 8192 && w->n_tiles16 <= (size_t)ctx->sm_count * 6 && smem <= 100 * 1024 &&
+         ((uintptr_t)x & 15) == 0;
+}
+
+template <int SEM, int MP>
+static int32_t gemv_quant_launch(rmi_ctx* ctx, const rmi_weight* w, const float* x, float* out, size_t out_stride) {
+  const size_t blocks = w->n_in / 32, smem = 128 + blocks * Q8_REC_BYTES + MP * (w->n_in + blocks * 4);
+  auto kern = q8_gemv_staged_kernel<SEM, MP, STAGED_QUANT>;
+  if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    rmi_set_error("cudaFuncSetAttribute(%zu B shared) failed", smem);
+    return RMI_ERR_CUDA;
+  }
+  const int pr = rmi_prof_begin(ctx, "q8_gemv");
+  const int32_t st = rmi_run(ctx, "q8_gemv_quant", kern, dim3((unsigned)w->n_tiles16, 1), dim3(128), smem, w->d_tile16, blocks,
+                             (const uint8_t*)nullptr, (const float*)nullptr, out, out_stride, (size_t)0, w->n_rows, (size_t)0,
+                             ctx->d_status, gemv_norm_args{x, nullptr, nullptr, nullptr, 0.0f}, ctx->fanout);
+  rmi_prof_end(ctx, pr);
+  return st;
+}
+
+template <int SEM>
+static int32_t gemv_quant_mp(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, float* out, size_t out_stride) {
+  return m == 1 ? gemv_quant_launch<SEM, 1>(ctx, w, x, out, out_stride)
+                : (m == 2 ? gemv_quant_launch<SEM, 2>(ctx, w, x, out, out_stride) : gemv_quant_launch<SEM, 4>(ctx, w, x, out, out_stride));
+}
+int32_t launch_q8_gemv_quant(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, float* out, size_t out_stride) {
+  switch (ctx->sem) {
+    case RMI_SEM_AVX2: return gemv_quant_mp<RMI_SEM_AVX2>(ctx, w, x, m, out, out_stride);
+    case RMI_SEM_NEON: return gemv_quant_mp<RMI_SEM_NEON>(ctx, w, x, m, out, out_stride);
+    default: return gemv_quant_mp<RMI_SEM_SCALAR>(ctx, w, x, m, out, out_stride);
+  }
+}
+
 template <int SEM, int MP>
 static int32_t gemv_fused_launch(rmi_ctx* ctx, const rmi_weight* w, const gemv_norm_args& na, float* out, size_t out_stride) {
   const size_t smem = gemv_fused_smem(w, MP), blocks = w->n_in / 32;
-  auto kern = q8_gemv_staged_kernel<SEM, MP, true>;
+  auto kern = q8_gemv_staged_kernel<SEM, MP, STAGED_NORM>;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
     rmi_set_error("cudaFuncSetAttribute(%zu B shared) failed", smem);
     return RMI_ERR_CUDA;
@@ -1178,9 +1253,6 @@ int32_t launch_silu_mul_quantize(rmi_ctx* ctx, const float* gate, const float* u
 int32_t launch_q8_matmul_f32(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, float* out) {
   if (m == 0 || w->n_rows == 0) return RMI_OK;
   const dim3 grid((unsigned)w->n_tiles16, (unsigned)m);
-  if (ctx->sem == RMI_SEM_AVX2)
-    q8_matmul_f32_kernel<RMI_SEM_AVX2><<<grid, 256, 0, ctx->stream>>>(w->d_tile16, w->n_in / 32, w->n_rows, x, out);
-  else
-    q8_matmul_f32_kernel<RMI_SEM_SCALAR><<<grid, 256, 0, ctx->stream>>>(w->d_tile16, w->n_in / 32, w->n_rows, x, out);
-  return rmi_post_launch(ctx, "q8_matmul_f32");
+  auto kern = ctx->sem == RMI_SEM_AVX2 ? q8_matmul_f32_kernel<RMI_SEM_AVX2> : q8_matmul_f32_kernel<RMI_SEM_SCALAR>;
+  return rmi_run(ctx, "q8_matmul_f32", kern, grid, dim3(256), 0, w->d_tile16, w->n_in / 32, w->n_rows, x, out);
 }
