@@ -411,6 +411,8 @@ static void free_weight(rmi_weight* w) {
   if (w->d_umma_gu_q) cudaFree(w->d_umma_gu_q);
   if (w->d_umma_gu_s) cudaFree(w->d_umma_gu_s);
   if (w->d_raw) cudaFree(w->d_raw);
+  if (w->d_q4k_q8k) cudaFree(w->d_q4k_q8k);
+  if (w->d_q4k_deq) cudaFree(w->d_q4k_deq);
   w->magic = 0;
   delete w;
 }
@@ -517,7 +519,7 @@ extern "C" int32_t rmi_weight_info(const rmi_weight* w, int32_t* ggml_type, size
   if (ggml_type) *ggml_type = w->ggml_type;
   if (n_in) *n_in = w->n_in;
   if (n_rows) *n_rows = w->n_rows;
-  if (device_bytes) *device_bytes = w->tile16_bytes + w->raw_bytes + w->umma_bytes;
+  if (device_bytes) *device_bytes = w->tile16_bytes + w->raw_bytes + w->umma_bytes + w->frag_bytes;
   return RMI_OK;
 }
 

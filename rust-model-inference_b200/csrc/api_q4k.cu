@@ -27,6 +27,27 @@ extern "C" int32_t rmi_quantize_q8_k(rmi_ctx* ctx, const float* x, size_t m, siz
   return RMI_OK;
 }
 
+// Quantize to Q8_K, then Q4_K x Q8_K; caller holds ctx->mu.  The tensor-core kernel takes over where the weights are no
+// longer what a call waits for; it exists for the AVX2 order only.
+static constexpr size_t Q4K_MMA_MIN_M = 16;
+
+static int32_t q4k_q8k_device(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, float* out, size_t row_begin, size_t row_end) {
+  if (m >= Q4K_MMA_MIN_M && ctx->sem == RMI_SEM_AVX2) {
+    uint8_t* xrec;
+    RMI_TRY(rmi_scratch(ctx, 0, q4k_mma_x_bytes(w, m, false), (void**)&xrec));
+    return launch_q4k_q8k_mma(ctx, w, x, m, xrec, out, row_begin, row_end);
+  }
+  const size_t n = w->n_in, nb = m * n / 256;
+  float* dd;
+  int8_t* dq;
+  int16_t* db;
+  RMI_TRY(rmi_scratch(ctx, 0, m * n, (void**)&dq));
+  RMI_TRY(rmi_scratch(ctx, 1, nb * 4, (void**)&dd));
+  RMI_TRY(rmi_scratch(ctx, 4, nb * 32, (void**)&db));
+  RMI_TRY(launch_q8k_quantize(ctx, x, m, n, dd, dq, db));
+  return launch_q4k_q8k_matmul(ctx, w, dd, dq, db, m, out, row_begin, row_end);
+}
+
 extern "C" int32_t rmi_matmul_q4_k_q8k(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, float* output,
                                        size_t row_begin, size_t row_end) {
   RMI_TRY(rmi_check_ctx(ctx));
@@ -37,17 +58,11 @@ extern "C" int32_t rmi_matmul_q4_k_q8k(rmi_ctx* ctx, const rmi_weight* w, const 
   RMI_REQUIRE(x && output, RMI_ERR_BAD_HANDLE, "rmi_matmul_q4_k_q8k: null buffer");
   RMI_REQUIRE(ctx->sem != RMI_SEM_NEON, RMI_ERR_UNSUPPORTED, "the reference has no NEON Q4_K x Q8_K kernel; use AVX2 or SCALAR");
   std::lock_guard<std::mutex> lock(ctx->mu);
-  const size_t n = w->n_in, nb = m * n / 256, nr = row_end - row_begin;
-  float *dx, *dd, *dout;
-  int8_t* dq;
-  int16_t* db;
+  const size_t n = w->n_in, nr = row_end - row_begin;
+  float *dx, *dout;
   RMI_TRY(host_in(ctx, x, m * n * 4, 5, true, (void**)&dx));
-  RMI_TRY(rmi_scratch(ctx, 0, m * n, (void**)&dq));
-  RMI_TRY(rmi_scratch(ctx, 1, nb * 4, (void**)&dd));
-  RMI_TRY(rmi_scratch(ctx, 4, nb * 32, (void**)&db));
   RMI_TRY(rmi_scratch(ctx, 6, m * w->n_rows * 4, (void**)&dout));
-  RMI_TRY(launch_q8k_quantize(ctx, dx, m, n, dd, dq, db));
-  RMI_TRY(launch_q4k_q8k_matmul(ctx, w, dd, dq, db, m, dout, row_begin, row_end));
+  RMI_TRY(q4k_q8k_device(ctx, w, dx, m, dout, row_begin, row_end));
   return host_out(ctx, output + row_begin, dout + row_begin, m, nr * 4, w->n_rows * 4);
 }
 
@@ -58,15 +73,14 @@ extern "C" int32_t rmi_matmul_q4_k_q8k_dev(rmi_ctx* ctx, const rmi_weight* w, co
   RMI_REQUIRE(x && output, RMI_ERR_BAD_HANDLE, "rmi_matmul_q4_k_q8k_dev: null buffer");
   RMI_REQUIRE(ctx->sem != RMI_SEM_NEON, RMI_ERR_UNSUPPORTED, "the reference has no NEON Q4_K x Q8_K kernel; use AVX2 or SCALAR");
   std::lock_guard<std::mutex> lock(ctx->mu);
-  const size_t n = w->n_in, nb = m * n / 256;
-  float* dd;
-  int8_t* dq;
-  int16_t* db;
-  RMI_TRY(rmi_scratch(ctx, 0, m * n, (void**)&dq));
-  RMI_TRY(rmi_scratch(ctx, 1, nb * 4, (void**)&dd));
-  RMI_TRY(rmi_scratch(ctx, 4, nb * 32, (void**)&db));
-  RMI_TRY(launch_q8k_quantize(ctx, x, m, n, dd, dq, db));
-  return launch_q4k_q8k_matmul(ctx, w, dd, dq, db, m, output, 0, w->n_rows);
+  return q4k_q8k_device(ctx, w, x, m, output, 0, w->n_rows);
+}
+
+static int32_t q4k_dequant_device(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, float* out) {
+  if (m < Q4K_MMA_MIN_M) return launch_q4k_dequant_matmul(ctx, w, x, m, out);
+  uint8_t* xrec;
+  RMI_TRY(rmi_scratch(ctx, 0, q4k_mma_x_bytes(w, m, true), (void**)&xrec));
+  return launch_q4k_dequant_mma(ctx, w, x, m, xrec, out);
 }
 
 extern "C" int32_t rmi_matmul_q4_k_dequant_dev(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m,
@@ -74,7 +88,8 @@ extern "C" int32_t rmi_matmul_q4_k_dequant_dev(rmi_ctx* ctx, const rmi_weight* w
   RMI_TRY(rmi_check_ctx(ctx));
   RMI_TRY(rmi_check_weight(w, RMI_GGML_Q4_K));
   RMI_REQUIRE(((uintptr_t)x & 15) == 0, RMI_ERR_BAD_SHAPE, "device input must be 16-byte aligned");
-  return launch_q4k_dequant_matmul(ctx, w, x, m, output);
+  std::lock_guard<std::mutex> lock(ctx->mu);
+  return q4k_dequant_device(ctx, w, x, m, output);
 }
 
 extern "C" int32_t rmi_matmul_q4_k_dequant(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, float* output) {
@@ -86,7 +101,7 @@ extern "C" int32_t rmi_matmul_q4_k_dequant(rmi_ctx* ctx, const rmi_weight* w, co
   float *dx, *dout;
   RMI_TRY(host_in(ctx, x, m * w->n_in * 4, 5, false, (void**)&dx));
   RMI_TRY(rmi_scratch(ctx, 6, m * w->n_rows * 4, (void**)&dout));
-  RMI_TRY(launch_q4k_dequant_matmul(ctx, w, dx, m, dout));
+  RMI_TRY(q4k_dequant_device(ctx, w, dx, m, dout));
   return host_out(ctx, output, dout, 1, m * w->n_rows * 4, 0);
 }
 

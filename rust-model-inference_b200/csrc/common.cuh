@@ -136,6 +136,8 @@ struct rmi_weight {
   size_t umma_bytes;
   uint8_t* d_raw;      // Q4_K
   size_t raw_bytes;
+  uint8_t *d_q4k_q8k, *d_q4k_deq;  // Q4_K records of the tensor-core paths (q4k_mma.cu), built on first use
+  size_t frag_bytes;
   // v-stack provenance (rows of a then rows of b); n_rows_a == 0 when not fused
   size_t n_rows_a;
 };

@@ -82,6 +82,11 @@ int32_t launch_q4k_q8k_matmul(rmi_ctx* ctx, const rmi_weight* w, const float* d8
                               size_t m, float* out, size_t row_begin, size_t row_end);
 int32_t launch_q4k_dequant_matmul(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, float* out);
 int32_t launch_q4k_dequantize(rmi_ctx* ctx, const rmi_weight* w, float* out);
+// q4k_mma.cu (tensor cores, many activation rows): f32 rows in, scratch of q4k_mma_x_bytes for their records
+size_t q4k_mma_x_bytes(const rmi_weight* w, size_t m, bool dequant);
+int32_t launch_q4k_q8k_mma(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, uint8_t* xrec, float* out, size_t row_begin,
+                           size_t row_end);
+int32_t launch_q4k_dequant_mma(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, uint8_t* xrec, float* out);
 
 // sharded.cu: 16-byte vectorised variant (falls back to the scalar kernel for unaligned shapes)
 int32_t launch_unshard_cols_vec(rmi_ctx* ctx, const float* gathered, size_t g, size_t m, size_t npr, float* out);
