@@ -65,7 +65,7 @@ enum { RMI_GGML_F32 = 0, RMI_GGML_F16 = 1, RMI_GGML_Q4_0 = 2, RMI_GGML_Q8_0 = 8,
  * quantizer (activation bytes and scale bits are those of q8_0.rs:176-230) and the exact block
  * sums, and accumulates whole blocks: each matmul's f32 output is within 1e-5 (max |a-b| /
  * max |ref|) of the eight-lane order on the same quantized input.  rmi_set_prefill_exact(ctx, 1)
- * keeps AVX2 calls of every size on the bit-exact CUDA-core kernels instead (slower).
+ * keeps AVX2 calls of every size in the bit-exact eight-lane order instead (slower).
  * Element-wise steps (rms_norm, rope, softmax, SiLU) follow the reference's portable x86 code
  * under all three settings; exp() is the correctly rounded f32 exponential. */
 typedef enum { RMI_SEM_AVX2 = 0, RMI_SEM_NEON = 1, RMI_SEM_SCALAR = 2 } rmi_semantics;
@@ -78,9 +78,9 @@ int32_t rmi_destroy(rmi_ctx* ctx);
 const char* rmi_last_error(void);
 int32_t rmi_set_semantics(rmi_ctx* ctx, int32_t sem);
 int32_t rmi_get_semantics(rmi_ctx* ctx, int32_t* sem);
-/* AVX2 semantics only (see above): on != 0 keeps calls of more than 32 rows on the CUDA-core kernels
+/* AVX2 semantics only (see above): on != 0 keeps calls of more than 32 rows in the eight-lane order
  * that reproduce matmul_q8_0_vs_q8_0_avx2 (src/ops/kernel/q8_0/avx2.rs:53-174) bit for bit; the
- * default (0) runs them on the tensor cores. */
+ * default (0) runs them in the faster whole-block order. */
 int32_t rmi_set_prefill_exact(rmi_ctx* ctx, int32_t on);
 /* Use an existing cudaStream_t (e.g. the framework's current stream); NULL restores the
  * context's own stream. */
@@ -317,8 +317,8 @@ int32_t rmi_session_set_forward(rmi_ctx* ctx, rmi_session* s, int32_t forward);
  *     (matmuls with M = positions, causal attention per position over the cache rows written on the way).
  *     Every operator of the reference's step works on one row and positions only meet in the K/V cache, so
  *     every cache row carries the bits of the reference's token loop (src/models/qwen3.rs:657-689): under
- *     NEON/SCALAR semantics the matmuls run on the tensor cores, under AVX2 on the bit-exact CUDA-core
- *     kernels.  Used for the default forward and prompts of 17 positions or more; otherwise the token loop.
+ *     NEON/SCALAR semantics the matmuls run on the tensor cores, under AVX2 in the bit-exact eight-lane
+ *     order.  Used for the default forward and prompts of 17 positions or more; otherwise the token loop.
  *   RMI_PREFILL_TOKEN_LOOP         one position per step, as the reference does.
  *   RMI_PREFILL_BATCHED_TENSOR     as BATCHED, but AVX2 semantics also take the tensor cores: cache rows are
  *     then within the 1e-5 matmul contract of the eight-lane order instead of bit-equal to it. */

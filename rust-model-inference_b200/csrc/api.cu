@@ -413,6 +413,7 @@ static void free_weight(rmi_weight* w) {
   if (w->d_raw) cudaFree(w->d_raw);
   if (w->d_q4k_q8k) cudaFree(w->d_q4k_q8k);
   if (w->d_q4k_deq) cudaFree(w->d_q4k_deq);
+  if (w->d_lanes) cudaFree(w->d_lanes);
   w->magic = 0;
   delete w;
 }
@@ -620,13 +621,13 @@ static bool use_tensor_cores(const rmi_ctx* ctx, size_t m) {
   // (avx2.rs:96-153), which the tensor core cannot deliver; for it the GEMM keeps the AVX2 quantizer
   // (activation bytes and scale bits unchanged), the exact block sums, and the whole-block chain,
   // whose f32 result is within 1e-5 of the eight-lane order.  rmi_set_prefill_exact(ctx, 1) keeps
-  // AVX2 calls of every m on the bit-exact CUDA-core kernels instead.
+  // AVX2 calls of every m in the bit-exact eight-lane order (q8_mma.cu, GEMV for few rows).
   return m > 32 && !(ctx->sem == RMI_SEM_AVX2 && ctx->prefill_exact);
 }
 
 // Plain matmuls (no fused epilogue) also take the tensor cores for 8 < m <= 32, with swapped operands,
-// where that is bit-exact (NEON and SCALAR); AVX2 calls of m <= 32 stay on the GEMV kernels, so the
-// decode path is bit-exact under every setting.
+// where that is bit-exact (NEON and SCALAR); AVX2 calls of m <= 32 keep the eight-lane order, so the decode path is
+// bit-exact under every setting.
 static bool matmul_on_tensor_cores(const rmi_ctx* ctx, size_t m) {
   if (use_tensor_cores(ctx, m)) return true;
   return m > 8 && m <= SWAP_AB_MAX_M && ctx->sem != RMI_SEM_AVX2;
@@ -697,6 +698,15 @@ extern "C" int32_t rmi_matmul_q8_0_prequantized(rmi_ctx* ctx, const rmi_weight* 
   return host_out(ctx, output + row_begin, dout + row_begin, m, nr * 4, n * 4);
 }
 
+// Scratch (slots slot, slot + 1) for m quantized rows that w is multiplied with.
+static int32_t rows_scratch(rmi_ctx* ctx, const rmi_weight* w, size_t m, int slot, q8_dst* d) {
+  const size_t blocks = w->n_in / 32;
+  *d = {nullptr, nullptr, q8_lanes_pack(ctx, w, m)};
+  if (d->pack >= 0) return rmi_scratch(ctx, slot, frag_x_bytes(m, blocks), (void**)&d->q8);
+  RMI_TRY(rmi_scratch(ctx, slot, m * w->n_in, (void**)&d->q8));
+  return rmi_scratch(ctx, slot + 1, m * blocks * 4, (void**)&d->scales);
+}
+
 // dout: [m][out_stride] f32, the weight's rows land in columns [0, n_rows); out_stride 0 = n_rows
 int32_t matmul_q8_0_device(rmi_ctx* ctx, const rmi_weight* w, const float* dx, size_t m, float* dout,
                            size_t out_stride, bool read_once) {
@@ -728,12 +738,10 @@ int32_t matmul_q8_0_device(rmi_ctx* ctx, const rmi_weight* w, const float* dx, s
     g.swap_ab = m <= SWAP_AB_MAX_M;
     return launch_gemm_tc(ctx, g);
   }
-  uint8_t* dq;
-  float* ds;
-  RMI_TRY(rmi_scratch(ctx, 0, m * w->n_in, (void**)&dq));
-  RMI_TRY(rmi_scratch(ctx, 1, m * blocks * 4, (void**)&ds));
-  RMI_TRY(launch_q8_quantize(ctx, dx, m, w->n_in, dq, ds, 0));
-  return launch_q8_gemv(ctx, w, dq, ds, m, dout, out_stride, 0, w->n_rows);
+  q8_dst x;
+  RMI_TRY(rows_scratch(ctx, w, m, 0, &x));
+  RMI_TRY(launch_q8_quantize(ctx, dx, m, w->n_in, x.q8, x.scales, x.pack < 0 ? 0 : 2, x.pack));
+  return launch_q8_rows(ctx, w, x, m, dout, out_stride);
 }
 
 extern "C" int32_t rmi_matmul_q8_0_fanout_dev(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m,
@@ -911,21 +919,19 @@ int32_t ffn_device(rmi_ctx* ctx, const rmi_weight* wgu, const rmi_weight* wd, co
     d.out_stride = n_embd;
     return launch_gemm_tc(ctx, d);
   }
-  uint8_t *q1, *q2;
-  float *sc1, *sc2, *gu;
-  RMI_TRY(rmi_scratch(ctx, 0, m * n_embd, (void**)&q1));
-  RMI_TRY(rmi_scratch(ctx, 1, m * b1 * 4, (void**)&sc1));
+  q8_dst x1, x2;
+  float* gu;
+  RMI_TRY(rows_scratch(ctx, wgu, m, 0, &x1));
   RMI_TRY(rmi_scratch(ctx, 2, m * 2 * n_ff * 4, (void**)&gu));
-  RMI_TRY(rmi_scratch(ctx, 3, m * n_ff, (void**)&q2));
-  RMI_TRY(rmi_scratch(ctx, 4, m * b2 * 4, (void**)&sc2));
+  RMI_TRY(rows_scratch(ctx, wd, m, 3, &x2));
   if (!read_once && q8_gemv_quant_eligible(ctx, wgu, dx, m)) {
     RMI_TRY(launch_q8_gemv_quant(ctx, wgu, dx, m, gu, 2 * n_ff));
   } else {
-    RMI_TRY(launch_q8_quantize(ctx, dx, m, n_embd, q1, sc1, 0));
-    RMI_TRY(launch_q8_gemv(ctx, wgu, q1, sc1, m, gu, 2 * n_ff, 0, 2 * n_ff));
+    RMI_TRY(launch_q8_quantize(ctx, dx, m, n_embd, x1.q8, x1.scales, x1.pack < 0 ? 0 : 2, x1.pack));
+    RMI_TRY(launch_q8_rows(ctx, wgu, x1, m, gu, 2 * n_ff));
   }
-  RMI_TRY(launch_silu_mul_quantize(ctx, gu, gu + n_ff, 2 * n_ff, m, n_ff, nullptr, q2, sc2));
-  return launch_q8_gemv(ctx, wd, q2, sc2, m, dout, n_embd, 0, n_embd);
+  RMI_TRY(launch_silu_mul_quantize(ctx, gu, gu + n_ff, 2 * n_ff, m, n_ff, nullptr, x2));
+  return launch_q8_rows(ctx, wd, x2, m, dout, n_embd);
 }
 
 extern "C" int32_t rmi_ffn_swiglu_q8_0_dev(rmi_ctx* ctx, const rmi_weight* wgu, const rmi_weight* wd,
@@ -1028,7 +1034,7 @@ extern "C" int32_t rmi_silu_mul(rmi_ctx* ctx, const float* gate, float* up, size
   RMI_CUDA_CHECK(cudaMemcpyAsync(du, up, n * 4, cudaMemcpyHostToDevice, ctx->stream));
   float* dact;
   RMI_TRY(rmi_scratch(ctx, 2, np * 4, (void**)&dact));
-  RMI_TRY(launch_silu_mul_quantize(ctx, dg, du, np, 1, np, dact, nullptr, nullptr));
+  RMI_TRY(launch_silu_mul_quantize(ctx, dg, du, np, 1, np, dact, {nullptr, nullptr, -1}));
   RMI_CUDA_CHECK(cudaMemcpyAsync(up, dact, n * 4, cudaMemcpyDeviceToHost, ctx->stream));
   RMI_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
   return RMI_OK;

@@ -134,10 +134,11 @@ struct rmi_weight {
   uint8_t* d_umma_gu_q;  // v-stacked gate|up weight in gate/up-interleaved row order (lazily built)
   float* d_umma_gu_s;
   size_t umma_bytes;
+  uint8_t* d_lanes;      // Q8_0, records of the eight-lane tensor-core matmul (q8_mma.cu), built on first use
   uint8_t* d_raw;      // Q4_K
   size_t raw_bytes;
   uint8_t *d_q4k_q8k, *d_q4k_deq;  // Q4_K records of the tensor-core paths (q4k_mma.cu), built on first use
-  size_t frag_bytes;
+  size_t frag_bytes;     // of the record layouts
   // v-stack provenance (rows of a then rows of b); n_rows_a == 0 when not fused
   size_t n_rows_a;
 };

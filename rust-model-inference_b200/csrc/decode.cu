@@ -13,6 +13,7 @@
 #include "decode.cuh"
 #include "decode_dev.cuh"
 #include "kernels.cuh"
+#include "q8_frag.cuh"
 
 namespace {
 
@@ -40,7 +41,7 @@ __global__ void embed_kernel(const uint8_t* __restrict__ emb, size_t blocks, con
 template <int SEM>
 __global__ void rmsnorm_quant_kernel(float* __restrict__ x, const float* __restrict__ add,
                                      const float* __restrict__ weight, size_t n, float eps,
-                                     uint8_t* __restrict__ q8, float* __restrict__ scales) {
+                                     const q8_dst dst) {
   __shared__ double s_part[8];
   __shared__ float s_scale;
   pdl_wait();
@@ -101,8 +102,8 @@ __global__ void rmsnorm_quant_kernel(float* __restrict__ x, const float* __restr
         for (int o = 16; o > 0; o >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
         float d, inv;
         q8_scale_pair<SEM>(a, &d, &inv);
-        q8[b * n + blk * 32 + lane] = (uint8_t)(int8_t)q8_quant_value<SEM>(v, inv);
-        if (lane == 0) scales[b * blocks + blk] = f16_round_trip(d);
+        store_q8_value(dst, blocks, b, blk, lane, q8_quant_value<SEM>(v, inv));
+        if (lane == 0) store_q8_scale(dst, blocks, b, blk, f16_round_trip(d));
       }
     }
   }
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(256)
     attention_kernel(const uint16_t* __restrict__ q16, uint16_t* __restrict__ k_cache,
                      uint16_t* __restrict__ v_cache, const int* __restrict__ d_step, size_t n_head,
                      size_t n_head_kv, size_t hd, size_t layer, size_t n_layer, size_t capacity, size_t chunk,
-                     float* __restrict__ attn_out, uint8_t* __restrict__ q8, float* __restrict__ scales,
+                     float* __restrict__ attn_out, const q8_dst dst,
                      const attn_fused_qk fq) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
@@ -346,8 +347,8 @@ __global__ void __launch_bounds__(256)
     for (int o = 16; o > 0; o >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
     float d, inv;
     q8_scale_pair<SEM>(a, &d, &inv);
-    q8[b * nq + out0 + blk * 32 + lane] = (uint8_t)(int8_t)q8_quant_value<SEM>(v, inv);
-    if (lane == 0) scales[b * (nq / 32) + (out0 / 32) + blk] = f16_round_trip(d);
+    store_q8_value(dst, nq / 32, b, out0 / 32 + blk, lane, q8_quant_value<SEM>(v, inv));
+    if (lane == 0) store_q8_scale(dst, nq / 32, b, out0 / 32 + blk, f16_round_trip(d));
   }
 }
 
@@ -379,7 +380,7 @@ __global__ void __launch_bounds__(G > 0 ? SEQ_THREADS_G : 256)
     attention_seq_kernel(const uint16_t* __restrict__ q16, const uint16_t* __restrict__ k_cache,
                          const uint16_t* __restrict__ v_cache, const int* __restrict__ d_step, size_t n_head,
                          size_t n_head_kv, size_t hd, size_t layer, size_t n_layer, size_t capacity,
-                         float* __restrict__ attn_out, uint8_t* __restrict__ q8, float* __restrict__ scales,
+                         float* __restrict__ attn_out, const q8_dst dst,
                          float* __restrict__ g_sc, double* __restrict__ g_pd) {
   extern __shared__ __align__(16) uint8_t smem[];
   pdl_wait();
@@ -613,8 +614,8 @@ __global__ void __launch_bounds__(G > 0 ? SEQ_THREADS_G : 256)
     for (int sft = 16; sft > 0; sft >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, sft));
     float dsc, inv;
     q8_scale_pair<SEM>(a, &dsc, &inv);
-    q8[b * nq + out0 + o] = (uint8_t)(int8_t)q8_quant_value<SEM>(v, inv);
-    if (lane == 0) scales[(b * nq + out0 + o) / 32] = f16_round_trip(dsc);
+    store_q8_value(dst, nq / 32, b, (out0 + o) / 32, lane, q8_quant_value<SEM>(v, inv));
+    if (lane == 0) store_q8_scale(dst, nq / 32, b, (out0 + o) / 32, f16_round_trip(dsc));
   }
 }
 
@@ -625,7 +626,7 @@ __global__ void __launch_bounds__(256)
     attention_online_kernel(const float* __restrict__ q32, const uint16_t* __restrict__ k_cache,
                             const uint16_t* __restrict__ v_cache, const int* __restrict__ d_step, size_t n_head,
                             size_t n_head_kv, size_t hd, size_t layer, size_t n_layer, size_t capacity,
-                            float* __restrict__ attn_out, uint8_t* __restrict__ q8, float* __restrict__ scales) {
+                            float* __restrict__ attn_out, const q8_dst dst) {
   constexpr int LN = SEM == RMI_SEM_AVX2 ? 8 : (SEM == RMI_SEM_NEON ? 4 : 1);
   extern __shared__ __align__(16) uint8_t smem[];
   pdl_wait();
@@ -741,8 +742,9 @@ __global__ void __launch_bounds__(256)
     for (int sft = 16; sft > 0; sft >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, sft));
     float dsc, inv;
     q8_scale_pair<SEM>(a, &dsc, &inv);
-    q8[o] = (uint8_t)(int8_t)q8_quant_value<SEM>(out, inv);
-    if (lane == 0) scales[o / 32] = f16_round_trip(dsc);
+    const size_t blk = (head * hd + tid) / 32;
+    store_q8_value(dst, nq / 32, b, blk, lane, q8_quant_value<SEM>(out, inv));
+    if (lane == 0) store_q8_scale(dst, nq / 32, b, blk, f16_round_trip(dsc));
   }
 }
 
@@ -774,7 +776,7 @@ __global__ void __launch_bounds__(256)
     attention_softmax_kernel(const float* __restrict__ q32, const typename kv_elem<KV16>::type* __restrict__ k_cache,
                              const typename kv_elem<KV16>::type* __restrict__ v_cache, const int* __restrict__ d_step,
                              size_t n_head, size_t n_head_kv, size_t hd, size_t layer, size_t n_layer, size_t capacity,
-                             float* __restrict__ attn_out, uint8_t* __restrict__ q8, float* __restrict__ scales) {
+                             float* __restrict__ attn_out, const q8_dst dst) {
   using kv_t = typename kv_elem<KV16>::type;
   constexpr int LN = SEM == RMI_SEM_AVX2 ? 8 : (SEM == RMI_SEM_NEON ? (KV16 ? 4 : 16) : 1);  // score lanes
   constexpr int LP = SEQ_PV ? 1 : LN;                                                        // chains per element
@@ -926,8 +928,9 @@ __global__ void __launch_bounds__(256)
     for (int sft = 16; sft > 0; sft >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, sft));
     float dsc, inv;
     q8_scale_pair<SEM>(a, &dsc, &inv);
-    q8[o] = (uint8_t)(int8_t)q8_quant_value<SEM>(out, inv);
-    if (lane == 0) scales[o / 32] = f16_round_trip(dsc);
+    const size_t blk = (head * hd + tid) / 32;
+    store_q8_value(dst, nq / 32, b, blk, lane, q8_quant_value<SEM>(out, inv));
+    if (lane == 0) store_q8_scale(dst, nq / 32, b, blk, f16_round_trip(dsc));
   }
 }
 
@@ -1050,11 +1053,11 @@ int32_t launch_embed(rmi_ctx* ctx, const rmi_weight* emb, const uint32_t* prompt
 }
 
 int32_t launch_rmsnorm_quant(rmi_ctx* ctx, float* x, const float* add, const float* weight, size_t n, float eps,
-                             uint8_t* q8, float* scales, size_t batch) {
+                             const q8_dst& dst, size_t batch) {
   auto kern = ctx->sem == RMI_SEM_AVX2 ? rmsnorm_quant_kernel<RMI_SEM_AVX2>
                                        : (ctx->sem == RMI_SEM_NEON ? rmsnorm_quant_kernel<RMI_SEM_NEON>
                                                                    : rmsnorm_quant_kernel<RMI_SEM_SCALAR>);
-  if (rmi_launch(ctx, kern, dim3((unsigned)batch), dim3(256), 0, x, add, weight, n, eps, q8, scales) != cudaSuccess) {
+  if (rmi_launch(ctx, kern, dim3((unsigned)batch), dim3(256), 0, x, add, weight, n, eps, dst) != cudaSuccess) {
     rmi_set_error("launch of rmsnorm_quant failed: %s", cudaGetErrorString(cudaGetLastError()));
     return RMI_ERR_CUDA;
   }
@@ -1093,8 +1096,7 @@ size_t attention_smem_bytes(const decode_dims& d) {
 }
 
 int32_t launch_attention(rmi_ctx* ctx, const decode_dims& d, const uint16_t* q16, uint16_t* k_cache,
-                         uint16_t* v_cache, const int* d_step, size_t layer, float* attn_out, uint8_t* q8,
-                         float* scales, const float* qkv, const float* q_norm, const float* k_norm,
+                         uint16_t* v_cache, const int* d_step, size_t layer, float* attn_out, const q8_dst& dst, const float* qkv, const float* q_norm, const float* k_norm,
                          const float* rope) {
   RMI_REQUIRE(d.hd % 8 == 0 && (d.n_head / d.n_head_kv) * d.hd % 32 == 0, RMI_ERR_UNSUPPORTED,
               "attention needs head_dim %% 8 == 0 and group*head_dim %% 32 == 0");
@@ -1102,7 +1104,7 @@ int32_t launch_attention(rmi_ctx* ctx, const decode_dims& d, const uint16_t* q16
   const unsigned cl = attention_cluster(d);
   const size_t chunk = (d.capacity + cl - 1) / cl;
   void (*kern)(const uint16_t*, uint16_t*, uint16_t*, const int*, size_t, size_t, size_t, size_t, size_t,
-               size_t, size_t, float*, uint8_t*, float*, const attn_fused_qk) =
+               size_t, size_t, float*, const q8_dst, const attn_fused_qk) =
       qkv ? (ctx->sem == RMI_SEM_AVX2 ? attention_kernel<RMI_SEM_AVX2, true>
                                       : (ctx->sem == RMI_SEM_NEON ? attention_kernel<RMI_SEM_NEON, true>
                                                                   : attention_kernel<RMI_SEM_SCALAR, true>))
@@ -1129,7 +1131,7 @@ int32_t launch_attention(rmi_ctx* ctx, const decode_dims& d, const uint16_t* q16
   cfg.attrs = attr;
   cfg.numAttrs = ctx->pdl ? 2 : 1;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, q16, k_cache, v_cache, d_step, d.n_head, d.n_head_kv, d.hd, layer,
-                                     d.n_layer, d.capacity, chunk, attn_out, q8, scales,
+                                     d.n_layer, d.capacity, chunk, attn_out, dst,
                                      attn_fused_qk{qkv, q_norm, k_norm, rope, d.eps});
   if (e != cudaSuccess) {
     rmi_set_error("attention launch failed: %s", cudaGetErrorString(e));
@@ -1161,7 +1163,7 @@ size_t attention_seq_scratch_bytes(const decode_dims& d) {
 }
 
 using attention_seq_fn = void (*)(const uint16_t*, const uint16_t*, const uint16_t*, const int*, size_t, size_t, size_t,
-                                 size_t, size_t, size_t, float*, uint8_t*, float*, float*, double*);
+                                 size_t, size_t, size_t, float*, const q8_dst, float*, double*);
 template <int SEM, bool GS>
 static attention_seq_fn attention_seq_pick_g(int g) {
   return g == 2 ? attention_seq_kernel<SEM, GS, 2> : (g == 4 ? attention_seq_kernel<SEM, GS, 4> : attention_seq_kernel<SEM, GS, 0>);
@@ -1177,8 +1179,7 @@ static attention_seq_fn attention_seq_pick(int sem, bool gs, int g) {
 }
 
 int32_t launch_attention_seq(rmi_ctx* ctx, const decode_dims& d, const uint16_t* q16, const uint16_t* k_cache,
-                             const uint16_t* v_cache, const int* d_step, size_t layer, float* attn_out, uint8_t* q8,
-                             float* scales, void* score_scratch) {
+                             const uint16_t* v_cache, const int* d_step, size_t layer, float* attn_out, const q8_dst& dst, void* score_scratch) {
   const size_t cs = (d.capacity + 7) & ~(size_t)7;
   const bool gs = score_scratch != nullptr;
   const size_t smem = attention_seq_smem_bytes(d, gs);
@@ -1193,7 +1194,7 @@ int32_t launch_attention_seq(rmi_ctx* ctx, const decode_dims& d, const uint16_t*
     return RMI_ERR_UNSUPPORTED;
   }
   if (rmi_launch(ctx, kern, dim3((unsigned)d.n_head_kv, (unsigned)d.batch), dim3(gv ? SEQ_THREADS_G : 256), smem, q16, k_cache, v_cache, d_step,
-                 d.n_head, d.n_head_kv, d.hd, layer, d.n_layer, d.capacity, attn_out, q8, scales, g_sc, g_pd) != cudaSuccess) {
+                 d.n_head, d.n_head_kv, d.hd, layer, d.n_layer, d.capacity, attn_out, dst, g_sc, g_pd) != cudaSuccess) {
     rmi_set_error("launch of attention_seq failed: %s", cudaGetErrorString(cudaGetLastError()));
     return RMI_ERR_CUDA;
   }
@@ -1202,8 +1203,7 @@ int32_t launch_attention_seq(rmi_ctx* ctx, const decode_dims& d, const uint16_t*
 
 // The CLI forward's attention: one CTA per (head, sequence).
 int32_t launch_attention_online(rmi_ctx* ctx, const decode_dims& d, const float* q32, const uint16_t* k_cache,
-                                const uint16_t* v_cache, const int* d_step, size_t layer, float* attn_out, uint8_t* q8,
-                                float* scales) {
+                                const uint16_t* v_cache, const int* d_step, size_t layer, float* attn_out, const q8_dst& dst) {
   RMI_REQUIRE(d.hd % 32 == 0 && d.hd <= 256, RMI_ERR_UNSUPPORTED, "online attention needs head_dim %% 32 == 0 and <= 256");
   const size_t smem = (2 * ((d.capacity + 3) & ~(size_t)3) + d.hd + 256) * 4 + 2 * ATT_TILE * d.hd * 2;
   auto kern = ctx->sem == RMI_SEM_AVX2 ? attention_online_kernel<RMI_SEM_AVX2>
@@ -1215,7 +1215,7 @@ int32_t launch_attention_online(rmi_ctx* ctx, const decode_dims& d, const float*
     return RMI_ERR_UNSUPPORTED;
   }
   if (rmi_launch(ctx, kern, dim3((unsigned)d.n_head, (unsigned)d.batch), dim3(256), smem, q32, k_cache, v_cache, d_step,
-                 d.n_head, d.n_head_kv, d.hd, layer, d.n_layer, d.capacity, attn_out, q8, scales) != cudaSuccess) {
+                 d.n_head, d.n_head_kv, d.hd, layer, d.n_layer, d.capacity, attn_out, dst) != cudaSuccess) {
     rmi_set_error("launch of attention_online failed: %s", cudaGetErrorString(cudaGetLastError()));
     return RMI_ERR_CUDA;
   }
@@ -1226,7 +1226,7 @@ template <bool KV16, bool SEQ_PV>
 static int32_t launch_attention_softmax_t(rmi_ctx* ctx, const decode_dims& d, const float* q32,
                                           const typename kv_elem<KV16>::type* k_cache,
                                           const typename kv_elem<KV16>::type* v_cache, const int* d_step, size_t layer,
-                                          float* attn_out, uint8_t* q8, float* scales) {
+                                          float* attn_out, const q8_dst& dst) {
   RMI_REQUIRE(d.hd % 32 == 0 && d.hd <= 256, RMI_ERR_UNSUPPORTED, "score-buffer attention needs head_dim %% 32 == 0 and <= 256");
   const size_t smem = (((d.capacity + 3) & ~(size_t)3) + d.hd + 16 * d.hd + 32) * 4 +
                       2 * SM_TILE * (d.hd * sizeof(typename kv_elem<KV16>::type) + 16);
@@ -1239,7 +1239,7 @@ static int32_t launch_attention_softmax_t(rmi_ctx* ctx, const decode_dims& d, co
     return RMI_ERR_UNSUPPORTED;
   }
   if (rmi_launch(ctx, kern, dim3((unsigned)d.n_head, (unsigned)d.batch), dim3(256), smem, q32, k_cache, v_cache, d_step,
-                 d.n_head, d.n_head_kv, d.hd, layer, d.n_layer, d.capacity, attn_out, q8, scales) != cudaSuccess) {
+                 d.n_head, d.n_head_kv, d.hd, layer, d.n_layer, d.capacity, attn_out, dst) != cudaSuccess) {
     rmi_set_error("launch of attention_softmax failed: %s", cudaGetErrorString(cudaGetLastError()));
     return RMI_ERR_CUDA;
   }
@@ -1247,17 +1247,16 @@ static int32_t launch_attention_softmax_t(rmi_ctx* ctx, const decode_dims& d, co
 }
 
 int32_t launch_attention_f32kv(rmi_ctx* ctx, const decode_dims& d, const float* q32, const float* k_cache,
-                               const float* v_cache, const int* d_step, size_t layer, float* attn_out, uint8_t* q8,
-                               float* scales, bool sequential_pv) {
+                               const float* v_cache, const int* d_step, size_t layer, float* attn_out, const q8_dst& dst, bool sequential_pv) {
   return sequential_pv
-             ? launch_attention_softmax_t<false, true>(ctx, d, q32, k_cache, v_cache, d_step, layer, attn_out, q8, scales)
-             : launch_attention_softmax_t<false, false>(ctx, d, q32, k_cache, v_cache, d_step, layer, attn_out, q8, scales);
+             ? launch_attention_softmax_t<false, true>(ctx, d, q32, k_cache, v_cache, d_step, layer, attn_out, dst)
+             : launch_attention_softmax_t<false, false>(ctx, d, q32, k_cache, v_cache, d_step, layer, attn_out, dst);
 }
 
 int32_t launch_attention_scores_f16kv(rmi_ctx* ctx, const decode_dims& d, const float* q32, const uint16_t* k_cache,
                                       const uint16_t* v_cache, const int* d_step, size_t layer, float* attn_out,
-                                      uint8_t* q8, float* scales) {
-  return launch_attention_softmax_t<true, true>(ctx, d, q32, k_cache, v_cache, d_step, layer, attn_out, q8, scales);
+                                      const q8_dst& dst) {
+  return launch_attention_softmax_t<true, true>(ctx, d, q32, k_cache, v_cache, d_step, layer, attn_out, dst);
 }
 
 size_t cli_attention_smem_bytes(const decode_dims& d, int forward) {

@@ -1,12 +1,13 @@
 // Launchers shared between translation units of librmi_cuda.so.
 #pragma once
 #include "common.cuh"
+#include "q8_frag.cuh"
 
 // q8_0.cu
 int32_t launch_q8_repack_tile16(rmi_ctx* ctx, const uint8_t* raw, uint8_t* dst, size_t n_rows, size_t blocks);
 int32_t launch_q8_copy_rows_tile16(rmi_ctx* ctx, const uint8_t* src, uint8_t* dst, size_t n_rows, size_t blocks, size_t row_off);
 int32_t launch_q8_build_umma(rmi_ctx* ctx, const uint8_t* t16, uint8_t* uq, float* us, size_t n_rows, size_t blocks, size_t n_ff_perm);
-int32_t launch_q8_quantize(rmi_ctx* ctx, const float* x, size_t m, size_t n, uint8_t* q8, float* scales, int out_mode);
+int32_t launch_q8_quantize(rmi_ctx* ctx, const float* x, size_t m, size_t n, uint8_t* q8, float* scales, int out_mode, int pack = 0);
 int32_t launch_q8_gemv(rmi_ctx* ctx, const rmi_weight* w, const uint8_t* xq, const float* xs, size_t m,
                        float* out, size_t out_stride, size_t row_begin, size_t row_end);
 // quantize + GEMV in one kernel for few f32 rows
@@ -19,7 +20,12 @@ int32_t launch_q8_gemv_fused_norm(rmi_ctx* ctx, const rmi_weight* w, const float
                                   const float* norm_w, float eps, float* x_out, size_t m, float* out, size_t out_stride);
 int32_t launch_q8_block_sums(rmi_ctx* ctx, const rmi_weight* w, const uint8_t* xq, size_t m, int32_t* sums);
 int32_t launch_silu_mul_quantize(rmi_ctx* ctx, const float* gate, const float* up, size_t in_stride, size_t m,
-                                 size_t n_ff, float* act, uint8_t* q8, float* scales);
+                                 size_t n_ff, float* act, const q8_dst& dst);
+
+// q8_mma.cu (tensor cores, AVX2 eight-lane order, bit-exact).  q8_lanes_pack: dst.pack for the quantizer of m rows that w
+// is multiplied with; -1 (row-major) where the GEMV kernels run.  Builds the weight's records on first use.
+int q8_lanes_pack(rmi_ctx* ctx, const rmi_weight* w, size_t m);
+int32_t launch_q8_rows(rmi_ctx* ctx, const rmi_weight* w, const q8_dst& x, size_t m, float* out, size_t out_stride);
 
 // gemm_tc.cu (tcgen05 int8 MMA)
 enum { GEMM_EPI_F32 = 0, GEMM_EPI_SWIGLU_Q8 = 1, GEMM_EPI_BLOCK_SUMS = 2 };

@@ -7,6 +7,7 @@
 //   hsum       src/ops/dot.rs:447-456
 #include "common.cuh"
 #include "kernels.cuh"
+#include "q8_frag.cuh"
 
 // ---------------------------------------------------------------- weight re-layout
 
@@ -77,13 +78,14 @@ __global__ void q8_build_umma_kernel(const uint8_t* __restrict__ t16, uint8_t* _
 
 // Eight threads per 32-block, thread L the four values 4L..4L+3 (one 16-byte load, one 4-byte store).
 // out_mode 0: q8 row-major [m][n], scales [m][n/32].
+// out_mode 2: activation records of the tensor-core matmul in the eight-lane order, 2^pack groups together.
 // out_mode 1: q8 in tcgen05 A-operand images ([tile128][slab][16 KiB]) and scales
 // [tile128][block][128]; rows m..pad are written as zeros by the caller's memset.
 // aligned: x on a 16-byte boundary and q8 on a 4-byte boundary; otherwise single elements are moved.
 template <int SEM>
 __global__ void __launch_bounds__(256)
     q8_quantize_kernel(const float* __restrict__ x, size_t n_words, size_t blocks, uint8_t* __restrict__ q8,
-                       float* __restrict__ scales, int out_mode, int aligned) {
+                       float* __restrict__ scales, int out_mode, int pack, int aligned) {
   pdl_wait();               // x may come from the preceding kernel of a dependent launch
   pdl_launch_dependents();
   const size_t word = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -113,6 +115,10 @@ __global__ void __launch_bounds__(256)
       for (int k = 0; k < 4; k++) q8[4 * word + k] = (uint8_t)(packed >> (8 * k));
     }
     if (L == 0) scales[blk] = sc;
+  } else if (out_mode == 2) {
+    const q8_dst dst = {q8, nullptr, pack};
+    store_q8_word(dst, blocks, row, b, L, q[0], q[1], q[2], q[3]);
+    if (L == 0) store_q8_scale(dst, blocks, row, b, sc);
   } else {
     const size_t n_slabs = (blocks + 3) / 4, tile = row / 128, r = row % 128, k = b * 32 + 4 * L;
     const size_t slab = k / 128, c = (k % 128) / 16, byte = k % 16;
@@ -863,8 +869,7 @@ __global__ void q8_block_sums_kernel(const uint8_t* __restrict__ w, size_t block
 template <int SEM>
 __global__ void silu_mul_quantize_kernel(const float* __restrict__ gate, const float* __restrict__ up,
                                          size_t in_stride, size_t m, size_t n_ff,
-                                         float* __restrict__ act, uint8_t* __restrict__ q8,
-                                         float* __restrict__ scales) {
+                                         float* __restrict__ act, const q8_dst dst) {
   pdl_wait();
   pdl_launch_dependents();
   size_t blocks = n_ff / 32;
@@ -877,14 +882,14 @@ __global__ void silu_mul_quantize_kernel(const float* __restrict__ gate, const f
   float s = __fdiv_rn(g, __fadd_rn(1.0f, exp_cr(-g)));
   float v = __fmul_rn(u, s);
   if (act) act[row * n_ff + b * 32 + lane] = v;
-  if (q8) {
+  if (dst.q8) {
     float a = fabsf(v);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
     float d, inv;
     q8_scale_pair<SEM>(a, &d, &inv);
-    q8[row * n_ff + b * 32 + lane] = (uint8_t)(int8_t)q8_quant_value<SEM>(v, inv);
-    if (lane == 0) scales[row * blocks + b] = f16_round_trip(d);
+    store_q8_value(dst, blocks, row, b, lane, q8_quant_value<SEM>(v, inv));
+    if (lane == 0) store_q8_scale(dst, blocks, row, b, f16_round_trip(d));
   }
 }
 
@@ -965,14 +970,14 @@ int32_t launch_q8_build_umma(rmi_ctx* ctx, const uint8_t* t16, uint8_t* uq, floa
 }
 
 int32_t launch_q8_quantize(rmi_ctx* ctx, const float* x, size_t m, size_t n, uint8_t* q8, float* scales,
-                           int out_mode) {
+                           int out_mode, int pack) {
   const size_t words = m * (n / 4);
   if (words == 0) return RMI_OK;
   auto kern = ctx->sem == RMI_SEM_AVX2 ? q8_quantize_kernel<RMI_SEM_AVX2>
                                        : (ctx->sem == RMI_SEM_NEON ? q8_quantize_kernel<RMI_SEM_NEON> : q8_quantize_kernel<RMI_SEM_SCALAR>);
   const int aligned = ((uintptr_t)x & 15) == 0 && ((uintptr_t)q8 & 3) == 0;
   return rmi_run(ctx, "q8_quantize", kern, dim3((unsigned)((words + 255) / 256)), dim3(256), 0, x, words, n / 32, q8, scales, out_mode,
-                 aligned);
+                 pack, aligned);
 }
 
 template <int SEM, int LB, int MP>
@@ -1236,14 +1241,14 @@ int32_t launch_q8_block_sums(rmi_ctx* ctx, const rmi_weight* w, const uint8_t* x
 }
 
 int32_t launch_silu_mul_quantize(rmi_ctx* ctx, const float* gate, const float* up, size_t in_stride,
-                                 size_t m, size_t n_ff, float* act, uint8_t* q8, float* scales) {
+                                 size_t m, size_t n_ff, float* act, const q8_dst& dst) {
   size_t warps = m * (n_ff / 32);
   if (warps == 0) return RMI_OK;
   unsigned grid = (unsigned)((warps + 7) / 8);
   auto kern = ctx->sem == RMI_SEM_AVX2 ? silu_mul_quantize_kernel<RMI_SEM_AVX2>
                                        : (ctx->sem == RMI_SEM_NEON ? silu_mul_quantize_kernel<RMI_SEM_NEON>
                                                                    : silu_mul_quantize_kernel<RMI_SEM_SCALAR>);
-  if (rmi_launch(ctx, kern, dim3(grid), dim3(256), 0, gate, up, in_stride, m, n_ff, act, q8, scales) != cudaSuccess) {
+  if (rmi_launch(ctx, kern, dim3(grid), dim3(256), 0, gate, up, in_stride, m, n_ff, act, dst) != cudaSuccess) {
     rmi_set_error("launch of silu_mul_quantize failed: %s", cudaGetErrorString(cudaGetLastError()));
     return RMI_ERR_CUDA;
   }

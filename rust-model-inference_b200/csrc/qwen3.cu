@@ -398,7 +398,7 @@ extern "C" int32_t rmi_session_create(rmi_ctx* ctx, const rmi_qwen3* model, size
   SESSION_ALLOC(s->logits, batch * d.vocab * 4);
   SESSION_ALLOC(s->rope, capacity * d.hd * 4);
   SESSION_ALLOC(s->q16, batch * nq * 2);
-  SESSION_ALLOC(s->q8, batch * max_n_in);
+  SESSION_ALLOC(s->q8, std::max(batch * max_n_in, frag_x_bytes(batch, max_n_in / 32)));
   SESSION_ALLOC(s->xs, batch * (max_n_in / 32) * 4);
   SESSION_ALLOC(s->d_step, 4);
   SESSION_ALLOC(s->d_flag, 4);
@@ -447,65 +447,71 @@ static int32_t enqueue_step(rmi_ctx* ctx, rmi_session* s, size_t n_prompt, size_
   const decode_dims& d = s->d;
   const size_t B = d.batch, nq = d.n_head * d.hd, nk = d.n_head_kv * d.hd;
   RMI_TRY(launch_embed(ctx, m->token_embd, s->prompts, n_prompt, s->gen, n_gen, s->d_step, s->x, B));
+  // where a step's quantizers leave the rows that w is multiplied with
+  auto rows_of = [&](const rmi_weight* w) { return q8_dst{s->q8, s->xs, q8_lanes_pack(ctx, w, B)}; };
   const float* pending = nullptr;  // residual branch still to be added to x
   float* xc = s->x;                  // current residual stream (ping-pongs with x2 on the fused path)
   float* xn = s->x2;
   for (size_t l = 0; l < d.n_layer; l++) {
     const layer_weights& w = m->layers[l];
+    const q8_dst x_attn = rows_of(w.wo), x_ff = rows_of(w.wdown);
     if (s->fused_norm) {
       // residual add + rms_norm + quantize happen inside the GEMV's prologue; it writes the updated x to xn
       RMI_TRY(launch_q8_gemv_fused_norm(ctx, w.wqkv, xc, pending, w.attn_norm, d.eps, xn, B, s->qkv, nq + 2 * nk));
       std::swap(xc, xn);
     } else {
-      RMI_TRY(launch_rmsnorm_quant(ctx, xc, pending, w.attn_norm, d.n_embd, d.eps, s->q8, s->xs, B));
-      RMI_TRY(launch_q8_gemv(ctx, w.wqkv, s->q8, s->xs, B, s->qkv, nq + 2 * nk, 0, nq + 2 * nk));
+      const q8_dst x = rows_of(w.wqkv);
+      RMI_TRY(launch_rmsnorm_quant(ctx, xc, pending, w.attn_norm, d.n_embd, d.eps, x, B));
+      RMI_TRY(launch_q8_rows(ctx, w.wqkv, x, B, s->qkv, nq + 2 * nk));
     }
     if (uses_f32_cache(s->forward)) {
       // src/app/text.rs:393-405, :458-496: f32 query and F32 cache, padded soft-max, one dot per output element;
       // src/app/logits.rs:513-560: the same scores and soft-max, then a sequential chain per output element
       RMI_TRY(launch_qk_norm_rope_kv(ctx, d, s->qkv, w.q_norm, w.k_norm, s->rope, s->d_step, s->q16, s->k_cache,
                                      s->v_cache, l, s->q32, s->k32_cache, s->v32_cache));
-      RMI_TRY(launch_attention_f32kv(ctx, d, s->q32, s->k32_cache, s->v32_cache, s->d_step, l, s->attn_dbg, s->q8, s->xs,
+      RMI_TRY(launch_attention_f32kv(ctx, d, s->q32, s->k32_cache, s->v32_cache, s->d_step, l, s->attn_dbg, x_attn,
                                      s->forward == RMI_FORWARD_APP_LOGITS_F32KV));
     } else if (s->forward == RMI_FORWARD_APP_LOGITS) {
       // src/app/logits.rs:474-512: f32 query x F16 cache scores, soft-max, sequential chain per output element
       RMI_TRY(launch_qk_norm_rope_kv(ctx, d, s->qkv, w.q_norm, w.k_norm, s->rope, s->d_step, s->q16, s->k_cache,
                                      s->v_cache, l, s->q32));
-      RMI_TRY(launch_attention_scores_f16kv(ctx, d, s->q32, s->k_cache, s->v_cache, s->d_step, l, s->attn_dbg, s->q8, s->xs));
+      RMI_TRY(launch_attention_scores_f16kv(ctx, d, s->q32, s->k_cache, s->v_cache, s->d_step, l, s->attn_dbg, x_attn));
     } else if (s->forward == RMI_FORWARD_APP_TEXT) {
       // src/app/text.rs:257-648: f32 query, online soft-max over the F16 cache
       RMI_TRY(launch_qk_norm_rope_kv(ctx, d, s->qkv, w.q_norm, w.k_norm, s->rope, s->d_step, s->q16, s->k_cache,
                                      s->v_cache, l, s->q32));
-      RMI_TRY(launch_attention_online(ctx, d, s->q32, s->k_cache, s->v_cache, s->d_step, l, s->attn_dbg, s->q8, s->xs));
+      RMI_TRY(launch_attention_online(ctx, d, s->q32, s->k_cache, s->v_cache, s->d_step, l, s->attn_dbg, x_attn));
     } else if (s->fused_qk) {
       // q/k norm, rotation and the cache write happen inside the attention kernel
-      RMI_TRY(launch_attention(ctx, d, s->q16, s->k_cache, s->v_cache, s->d_step, l, s->attn_dbg, s->q8, s->xs, s->qkv,
+      RMI_TRY(launch_attention(ctx, d, s->q16, s->k_cache, s->v_cache, s->d_step, l, s->attn_dbg, x_attn, s->qkv,
                                w.q_norm, w.k_norm, s->rope));
     } else {
       RMI_TRY(launch_qk_norm_rope_kv(ctx, d, s->qkv, w.q_norm, w.k_norm, s->rope, s->d_step, s->q16, s->k_cache,
                                      s->v_cache, l));
       if (s->seq_attention)
-        RMI_TRY(launch_attention_seq(ctx, d, s->q16, s->k_cache, s->v_cache, s->d_step, l, s->attn_dbg, s->q8, s->xs, s->attn_scratch));
+        RMI_TRY(launch_attention_seq(ctx, d, s->q16, s->k_cache, s->v_cache, s->d_step, l, s->attn_dbg, x_attn, s->attn_scratch));
       else
-        RMI_TRY(launch_attention(ctx, d, s->q16, s->k_cache, s->v_cache, s->d_step, l, s->attn_dbg, s->q8, s->xs));
+        RMI_TRY(launch_attention(ctx, d, s->q16, s->k_cache, s->v_cache, s->d_step, l, s->attn_dbg, x_attn));
     }
-    RMI_TRY(launch_q8_gemv(ctx, w.wo, s->q8, s->xs, B, s->proj, d.n_embd, 0, d.n_embd));
+    RMI_TRY(launch_q8_rows(ctx, w.wo, x_attn, B, s->proj, d.n_embd));
     if (s->fused_norm) {
       RMI_TRY(launch_q8_gemv_fused_norm(ctx, w.wgu, xc, s->proj, w.ffn_norm, d.eps, xn, B, s->gu, 2 * d.n_ff));
       std::swap(xc, xn);
     } else {
-      RMI_TRY(launch_rmsnorm_quant(ctx, xc, s->proj, w.ffn_norm, d.n_embd, d.eps, s->q8, s->xs, B));
-      RMI_TRY(launch_q8_gemv(ctx, w.wgu, s->q8, s->xs, B, s->gu, 2 * d.n_ff, 0, 2 * d.n_ff));
+      const q8_dst x = rows_of(w.wgu);
+      RMI_TRY(launch_rmsnorm_quant(ctx, xc, s->proj, w.ffn_norm, d.n_embd, d.eps, x, B));
+      RMI_TRY(launch_q8_rows(ctx, w.wgu, x, B, s->gu, 2 * d.n_ff));
     }
-    RMI_TRY(launch_silu_mul_quantize(ctx, s->gu, s->gu + d.n_ff, 2 * d.n_ff, B, d.n_ff, nullptr, s->q8, s->xs));
-    RMI_TRY(launch_q8_gemv(ctx, w.wdown, s->q8, s->xs, B, s->proj, d.n_embd, 0, d.n_embd));
+    RMI_TRY(launch_silu_mul_quantize(ctx, s->gu, s->gu + d.n_ff, 2 * d.n_ff, B, d.n_ff, nullptr, x_ff));
+    RMI_TRY(launch_q8_rows(ctx, w.wdown, x_ff, B, s->proj, d.n_embd));
     pending = s->proj;
   }
   // x += last down projection; output norm; logits; greedy token.  After an even number of swaps the
   // stream is back in s->x, which is what rmi_session_read_hidden returns.
-  RMI_TRY(launch_rmsnorm_quant(ctx, xc, pending, m->output_norm, d.n_embd, d.eps, s->q8, s->xs, B));
+  const q8_dst x_out = rows_of(m->output);
+  RMI_TRY(launch_rmsnorm_quant(ctx, xc, pending, m->output_norm, d.n_embd, d.eps, x_out, B));
   if (with_logits) {
-    RMI_TRY(launch_q8_gemv(ctx, m->output, s->q8, s->xs, B, s->logits, d.vocab, 0, d.vocab));
+    RMI_TRY(launch_q8_rows(ctx, m->output, x_out, B, s->logits, d.vocab));
     RMI_TRY(launch_argmax(ctx, s->logits, d.vocab, s->d_step, n_prompt, s->gen, n_gen, s->d_flag, B, s->argmax_v, s->argmax_i,
                           s->forward == RMI_FORWARD_APP_TEXT || s->forward == RMI_FORWARD_APP_TEXT_F32KV));
   }
@@ -517,12 +523,16 @@ static int32_t build_graphs(rmi_ctx* ctx, rmi_session* s, size_t n_prompt, size_
       s->graph_stream == ctx->stream)
     return RMI_OK;
   drop_graphs(s);
+  for (const auto& l : s->model->layers)   // weight records are built outside the capture
+    for (const rmi_weight* w : {l.wqkv, l.wo, l.wgu, l.wdown}) (void)q8_lanes_pack(ctx, w, s->d.batch);
+  (void)q8_lanes_pack(ctx, s->model->output, s->d.batch);
   for (int which = 0; which < 2; which++) {
     RMI_CUDA_CHECK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     // programmatic dependent launch along the step's kernel chain: the next kernel's weight copy
-    // overlaps the tail of the current one.  Measured gain for small batches only (large grids lose).
+    // overlaps the tail of the current one.  Measured on the 0.6B step: +6 % at batch 8 and +5 % at batch 24 and 32;
+    // with the GEMV kernels, whose grids are large, +3 % at 16 and -8 % at 32.
     const bool pdl_before = ctx->pdl;
-    ctx->pdl = s->d.batch <= 16;  // measured on the 0.6B step: +6 % at batch 8, +3 % at 16, -8 % at 32
+    ctx->pdl = s->d.batch <= 16 || q8_lanes_pack(ctx, s->model->output, s->d.batch) >= 0;
     int32_t st = enqueue_step(ctx, s, n_prompt, n_gen, which == 1);
     ctx->pdl = pdl_before;
     cudaGraph_t g = nullptr;
@@ -620,9 +630,11 @@ static int32_t prepare_prefill(rmi_ctx* ctx, rmi_session* s, size_t P) {
   const size_t widest = nq > d.n_ff ? (nq > d.n_embd ? nq : d.n_embd) : (d.n_ff > d.n_embd ? d.n_ff : d.n_embd);
   const size_t rows_pad = (rows + 127) / 128 * 128, wide_pad = (widest + 127) / 128 * 128;
   void* unused;
-  RMI_TRY(rmi_scratch(ctx, 0, rows_pad * wide_pad, &unused));                 // quantized rows (row-major or images)
+  const bool lanes = !prefill_on_tensor_cores(ctx, s) && ctx->sem == RMI_SEM_AVX2;
+  const size_t x_bytes = lanes ? frag_x_bytes(rows, widest / 32) : rows_pad * wide_pad;
+  RMI_TRY(rmi_scratch(ctx, 0, x_bytes, &unused));                             // quantized rows (images or records)
   RMI_TRY(rmi_scratch(ctx, 1, rows_pad * (wide_pad / 32) * 4, &unused));      // their scales
-  RMI_TRY(rmi_scratch(ctx, 3, rows_pad * wide_pad, &unused));
+  RMI_TRY(rmi_scratch(ctx, 3, x_bytes, &unused));
   RMI_TRY(rmi_scratch(ctx, 4, rows_pad * (wide_pad / 32) * 4, &unused));
   if (prefill_on_tensor_cores(ctx, s)) {
     for (const auto& l : m->layers) {
@@ -632,7 +644,9 @@ static int32_t prepare_prefill(rmi_ctx* ctx, rmi_session* s, size_t P) {
       RMI_TRY(ensure_umma_layout(ctx, l.wdown));
     }
   } else {
-    RMI_TRY(rmi_scratch(ctx, 2, rows * 2 * d.n_ff * 4, &unused));             // gate | up rows of the CUDA-core FFN
+    RMI_TRY(rmi_scratch(ctx, 2, rows * 2 * d.n_ff * 4, &unused));             // gate | up rows
+    for (const auto& l : m->layers)
+      for (const rmi_weight* w : {l.wqkv, l.wo, l.wgu, l.wdown}) (void)q8_lanes_pack(ctx, w, rows);
   }
   return RMI_OK;
 }
@@ -643,7 +657,7 @@ static int32_t enqueue_prefill(rmi_ctx* ctx, rmi_session* s, size_t n_prompt, si
   const size_t nq = d.n_head * d.hd;
   const size_t group_seqs = prefill_group_seqs(s, P);
   RMI_TRY(ensure_prefill_buffers(s, group_seqs * P));
-  // AVX2 semantics: the eight-lane accumulation order is reproduced bit for bit by the CUDA-core kernels, which
+  // AVX2 semantics: the eight-lane accumulation order is reproduced bit for bit (q8_mma.cu), which
   // keeps every cache row identical to the token loop's; RMI_PREFILL_BATCHED_TENSOR trades that for the tensor cores
   const bool exact_before = ctx->prefill_exact;
   if (ctx->sem == RMI_SEM_AVX2) ctx->prefill_exact = s->prefill_mode != RMI_PREFILL_BATCHED_TENSOR;

@@ -1,0 +1,68 @@
+"""Edges of the kernels that a call's sizes select: tiles that are not full, remainders along K, the smallest and the
+largest sizes of a choice.  Bar: the bits of the CPU oracle."""
+import numpy as np
+import pytest
+
+from helpers import bits, rel_err
+from oracle import orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx(rmi):
+    c = rmi.context(0)
+    c.set_semantics(rmi.SEM_AVX2)
+    yield c
+    c.set_prefill_exact(False)
+
+
+# one shape at least for every CTA tile of the eight-lane tensor-core matmul (4, 8, 16, 32 activation rows), K of one
+# block, of a partial and of several chunks
+@pytest.mark.parametrize("m,n,k", [(5, 1, 32), (9, 130, 544), (17, 2555, 96), (31, 2560, 1056), (48, 6144, 64), (32, 6130, 160),
+                                   (150, 6159, 416)])
+def test_eight_lane_matmul_on_tensor_cores(rmi, ctx, m, n, k):
+    wb = rmi.synth.q8_0_weight(n, k, seed=m + k)
+    w = rmi.QuantizedTensor.from_bytes(wb, rmi.GGML_Q8_0, k, n)
+    x = rmi.synth.normal((m, k), seed=n)
+    x[m // 2] = 0.0
+    ctx.set_prefill_exact(True)
+    got = rmi.matmul_q8_0(w, x)
+    ctx.set_prefill_exact(False)
+    assert np.array_equal(bits(got), bits(orc.q8_forward_batched(wb, x, k, n, orc.SEM_AVX2, threads=8)))
+    w.free()
+
+
+# quantize and GEMV in one kernel (1, 2 and 4 rows up to its longest K), and the row counts around it
+@pytest.mark.parametrize("m,n,k", [(1, 1, 32), (1, 4097, 8192), (2, 100, 4096), (4, 33, 2048), (4, 16, 2080), (3, 48, 96)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_few_rows_from_device_pointers(rmi, ctx, m, n, k, offset):
+    torch = pytest.importorskip("torch")
+    wb = rmi.synth.q8_0_weight(n, k, seed=k)
+    w = rmi.QuantizedTensor.from_bytes(wb, rmi.GGML_Q8_0, k, n)
+    x = rmi.synth.normal((m, k), seed=m)
+    d = torch.zeros(m * k + 4, device="cuda")
+    d[offset:offset + m * k] = torch.from_numpy(x.reshape(-1)).cuda()      # on a 16-byte boundary, and off one
+    out = torch.empty(m * n, device="cuda")
+    torch.cuda.synchronize()
+    rmi.matmul_q8_0_dev(w, d.data_ptr() + 4 * offset, m, out.data_ptr())
+    ctx.sync()
+    assert np.array_equal(bits(out.cpu().numpy().reshape(m, n)), bits(orc.q8_forward_batched(wb, x, k, n, orc.SEM_AVX2)))
+    w.free()
+
+
+# Q4_0 and Q6_K through one trait call: row counts on both sides of the kernels' row tiles, ragged output rows
+@pytest.mark.parametrize("kind,m,n,k", [("q4_0", 1, 17, 32), ("q4_0", 7, 130, 96), ("q4_0", 8, 64, 1024), ("q4_0", 25, 33, 2080),
+                                        ("q6_k", 1, 1, 256), ("q6_k", 3, 37, 512), ("q6_k", 9, 16, 1024), ("q6_k", 2, 5000, 256)])
+def test_kernel_trait_forward_batched(rmi, ctx, kind, m, n, k):
+    wb = getattr(rmi.synth, kind + "_weight")(n, k, seed=n + k)
+    kern = (rmi.Q4_0Kernel if kind == "q4_0" else rmi.Q6_KKernel).new(wb, k, n)
+    x = rmi.synth.normal((m, k), seed=m)
+    got = np.full((m, n), np.nan, np.float32)
+    kern.forward_batched(x, got, k, n)
+    for t in range(m):
+        if kind == "q4_0":
+            ref = orc.q4_0_forward_prequantized(wb, *orc.quantize_q8_0(x[t], orc.SEM_AVX2), k, n)
+        else:
+            ref = orc.q6k_forward_prepared(wb, x[t], k, n)
+        assert np.array_equal(bits(got[t]), bits(ref)), t
