@@ -95,141 +95,178 @@ __global__ void qk_norm_rope_kv_rows_kernel(const float* __restrict__ qkv, size_
   norm_rope_head_f16(src, is_q ? q_norm : k_norm, eps, rope + p * hd, hd, lane, dst);
 }
 
-// Causal attention of QT consecutive query positions of one (sequence, kv head): the `group` query heads that
-// share the kv head are processed together, so a CTA owns QT * group query rows.  K and V stream through two
-// shared-memory tiles; the scores of all rows stay in shared memory (row stride = positions visible to the last
-// query of the CTA).  Per row the arithmetic is that of one decode step: sequential f64 dot over the head
-// dimension, f32 score * 1/sqrt(hd), max, exp, sequential f32 sum over the positions, divide, f16, then per
-// output element the f64 sum over the positions in ascending order.
-constexpr int PF_TILE = 64;
+// Causal attention of up to eight query rows of one (sequence, kv head); row r of a kv head is query head r % group of the
+// group that shares it, at position r / group, so a CTA's rows are consecutive positions.  Per row the arithmetic is that
+// of one decode step: sequential f64 dot over the head dimension, f32 score * 1/sqrt(hd), max, exp, sequential f32 sum over
+// the positions, divide, f16, then per output element the f64 sum over the positions in ascending order.
+//
+// Bound: the f64 pipe, two multiply-adds per query row, visible position and head element (a conversion to f64 takes four
+// times as long as a multiply-add, so the products are not converted).  A product of two f16 values is exact, so a fused
+// multiply-add rounds as a multiplication and an addition would, and m8n8k4 f64 MMAs add their four products one after the
+// other in ascending order, each with one rounding (checked against chains of fma on operands of full precision: no bit
+// differs).  Multiply-add instructions of the CUDA cores run at 2.7 cycles instead of 2 on three 64-bit register operands
+// and need a load per four of them; an MMA is 16 cycles for 256 multiply-adds and one value per thread and operand.
+// Measured, 16 query and 8 kv heads of 128: 480 positions 225 -> 64 us, 960 positions 209 us (the MMAs alone: 26 and 104 us;
+// the rest is the soft-max, the f16 conversions and the staging of K and V, which four CTAs per SM overlap in part).
+// f16 -> f64 in integer instructions: of the f64 form only the high word is not zero, and with the exponent left 1008 too
+// small (2^1008 is put into the other factor; both exact) that word is the sign-extended f16 shifted and masked.
+constexpr int PF_THREADS = 128, PF_TILE = 64;
 
+__device__ __forceinline__ double f16_small_f64(int16_t bits) {   // x * 2^-1008 of the f16 value x, infinities and NaNs too
+  const int h = bits;
+  int hi = (int)(((uint32_t)h << 10) & 0x81ffffffu);
+  if ((~h & 0x7c00) == 0) hi |= 0x7ff00000;
+  return __hiloint2double(hi, 0);
+}
+__device__ __forceinline__ int f32_hi_large(float v) {          // high word of v * 2^1008 for f16-valued v; the low one is 0
+  return __double2hiint((double)v * 0x1p1008);
+}
+__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
+}
+
+// Four warps.  Scores: a warp takes every fourth 8-position tile, its rows of Q stay in registers.  Outputs: a warp takes
+// HD / 4 head elements.  K and V tiles of 64 positions stream through two buffers.
 template <int HD>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(PF_THREADS, 3)
     attention_prefill_kernel(const uint16_t* __restrict__ q16, const uint16_t* __restrict__ k_cache,
                              const uint16_t* __restrict__ v_cache, size_t n_head, size_t n_head_kv, size_t layer,
-                             size_t n_layer, size_t capacity, size_t P, size_t b0, int QT, float* __restrict__ attn_out) {
+                             size_t n_layer, size_t capacity, size_t P, size_t b0, size_t n_seq, int rows_per_cta,
+                             float* __restrict__ attn_out) {
+  constexpr int STRIDE = HD + 8, TILE = PF_TILE * STRIDE, NT = HD / 32;   // f16 row stride: rows four banks apart
   pdl_wait();
   pdl_launch_dependents();
-  extern __shared__ __align__(16) uint8_t smem[];
-  const size_t kvh = blockIdx.y, bl = blockIdx.z, b = b0 + bl;
-  const int t_first = (int)blockIdx.x * QT;
-  const int nqp = min(QT, (int)P - t_first);        // query positions of this CTA
-  const int t_last = t_first + nqp - 1;
-  const int T = t_last + 1;                          // cache positions any row of the CTA may see
+  extern __shared__ __align__(16) uint8_t pf_smem[];
+  int16_t* kv = reinterpret_cast<int16_t*>(pf_smem);               // 2 x [PF_TILE][STRIDE]
+  int* sc = reinterpret_cast<int*>(pf_smem + 2 * TILE * 2);         // [rows][cs] scores, exponentials (f32), high words of p * 2^1008
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = lane >> 2, c = lane & 3;
+  // the longest rows of every head and sequence start first, the shortest fill the gaps at the end
+  const size_t kvh = blockIdx.x % n_head_kv, bl = blockIdx.x / n_head_kv % n_seq, b = b0 + bl;
   const int group = (int)(n_head / n_head_kv);
-  const int rows = nqp * group;                      // row = qp * group + g
+  const int r0 = (int)((gridDim.x - 1 - blockIdx.x) / (n_head_kv * n_seq)) * rows_per_cta;
+  const int rows = min(rows_per_cta, (int)P * group - r0);
+  const int T = (r0 + rows - 1) / group + 1;                         // cache positions that any row may see
+  const int n_tiles = (T + PF_TILE - 1) / PF_TILE, cs = n_tiles * PF_TILE + 4;
   const size_t nq = n_head * HD, nk = n_head_kv * HD;
-  const size_t cs = ((size_t)T + 7) & ~(size_t)7;
-  float* sc = reinterpret_cast<float*>(smem);                                   // [QT*group][cs] scores, then weights
-  uint16_t* p16 = reinterpret_cast<uint16_t*>(sc + (size_t)QT * group * cs);    // [QT*group][cs]
-  uint16_t* qs = p16 + (size_t)QT * group * cs;                                 // [QT*group][HD + 2] (row stride of 65 words: conflict-free)
-  // 2 x PF_TILE x HD f16 tiles behind the query rows, on a 16-byte boundary
-  uint8_t* tiles = smem + (((size_t)(reinterpret_cast<uint8_t*>(qs + (size_t)QT * group * (HD + 2)) - smem) + 15) & ~(size_t)15);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr size_t row_bytes = HD * 2, tile_bytes = PF_TILE * row_bytes, row16 = HD / 8;
-  const int n_tiles = (T + PF_TILE - 1) / PF_TILE;
   const float kq_scale = __fdiv_rn(1.0f, __fsqrt_rn((float)HD));
   const uint16_t* kbase = k_cache + ((b * n_layer + layer) * capacity) * nk + kvh * HD;
   const uint16_t* vbase = v_cache + ((b * n_layer + layer) * capacity) * nk + kvh * HD;
-  auto stage = [&](const uint16_t* base, int tile, int buf) {
-    const int t0 = tile * PF_TILE, nt = min(PF_TILE, T - t0);
-    uint8_t* dst = tiles + (size_t)buf * tile_bytes;
-    for (size_t i = tid; i < (size_t)nt * row16; i += blockDim.x)
-      cp_async16(dst + (i / row16) * row_bytes + (i % row16) * 16, base + (size_t)(t0 + i / row16) * nk + (i % row16) * 8);
+  auto stage = [&](const uint16_t* base, int tile) {   // positions past T repeat the last one
+    int16_t* dst = kv + (tile & 1) * TILE;
+#pragma unroll
+    for (int u = 0; u < PF_TILE * HD / 8 / PF_THREADS; u++) {
+      const int i = tid + PF_THREADS * u, t = min(tile * PF_TILE + i / (HD / 8), T - 1);
+      cp_async16(dst + i / (HD / 8) * STRIDE + i % (HD / 8) * 8, base + (size_t)t * nk + i % (HD / 8) * 8);
+    }
     cp_async_commit();
   };
-  // query rows: q16 row (bl * P + t) holds all heads of position t
-  for (size_t i = tid; i < (size_t)rows * (HD / 2); i += blockDim.x) {
-    const int row = (int)(i / (HD / 2)), w = (int)(i % (HD / 2));
-    const int qp = row / group, g = row % group;
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(q16 + (bl * P + t_first + qp) * nq + (kvh * group + g) * HD);
-    reinterpret_cast<uint32_t*>(qs + (size_t)row * (HD + 2))[w] = src[w];
-  }
-  stage(kbase, 0, 0);
+  auto arrived = [&](bool more) {
+    if (more) cp_async_wait<1>(); else cp_async_wait<0>();
+    __syncthreads();
+  };
+  stage(kbase, 0);
+  const int fr = r0 + min(r, rows - 1), pos = r < rows ? fr / group : -1;   // this thread's row and its position
+  const size_t row_off = (bl * P + fr / group) * nq + (kvh * group + fr % group) * HD;
+
   // scores[row][t] = f32(sum_f64 q*k) * kq_scale for t <= position of the row (dot.rs:115-118)
-  for (int tile = 0; tile < n_tiles; tile++) {
-    if (tile + 1 < n_tiles) stage(kbase, tile + 1, (tile + 1) & 1);
-    if (tile + 1 < n_tiles) cp_async_wait<1>(); else cp_async_wait<0>();
-    __syncthreads();
-    const uint8_t* kt = tiles + (size_t)(tile & 1) * tile_bytes;
-    const int t0 = tile * PF_TILE, nt = min(PF_TILE, T - t0);
-    for (int item = tid; item < nt * rows; item += blockDim.x) {
-      const int tl = item / rows, row = item % rows;
-      const int t = t0 + tl, tq = t_first + row / group;
-      if (t > tq) continue;  // causal: a query sees positions 0..its own
-      const uint32_t* kr = reinterpret_cast<const uint32_t*>(kt + (size_t)tl * row_bytes);
-      const uint32_t* qr = reinterpret_cast<const uint32_t*>(qs + (size_t)row * (HD + 2));
-      double s = 0.0;
-#pragma unroll 8
-      for (int i = 0; i < HD / 2; i++) {
-        const uint32_t kk = kr[i], qq = qr[i];
-        s += (double)__fmul_rn(f16_bits_to_f32((uint16_t)(qq & 0xffff)), f16_bits_to_f32((uint16_t)(kk & 0xffff)));
-        s += (double)__fmul_rn(f16_bits_to_f32((uint16_t)(qq >> 16)), f16_bits_to_f32((uint16_t)(kk >> 16)));
+  {
+    int qh[HD / 4];
+#pragma unroll
+    for (int s = 0; s < HD / 4; s++) qh[s] = f32_hi_large(f16_bits_to_f32(q16[row_off + 4 * s + c]));
+    for (int tile = 0; tile < n_tiles; tile++) {
+      if (tile + 1 < n_tiles) stage(kbase, tile + 1);
+      arrived(tile + 1 < n_tiles);
+      const int16_t* kt = kv + (tile & 1) * TILE + (8 * warp + r) * STRIDE + c;
+      const int t0 = tile * PF_TILE + 8 * warp;   // this warp: positions t0 .. t0 + 7 and t0 + 32 .. t0 + 39
+      if (t0 < T) {
+        double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll
+        for (int s = 0; s < HD / 4; s++) {
+#pragma unroll
+          for (int n = 0; n < 2; n++) mma_f64(acc[n], __hiloint2double(qh[s], 0), f16_small_f64(kt[32 * n * STRIDE + 4 * s]));
+        }
+#pragma unroll
+        for (int n = 0; n < 2; n++)
+#pragma unroll
+          for (int e = 0; e < 2; e++) {
+            const int t = t0 + 32 * n + 2 * c + e;
+            if (t <= pos) sc[r * cs + t] = __float_as_int(__fmul_rn((float)acc[n][e], kq_scale));
+          }
       }
-      sc[(size_t)row * cs + t] = __fmul_rn((float)s, kq_scale);
+      __syncthreads();
     }
-    __syncthreads();
   }
-  stage(vbase, 0, 0);  // the first V tile travels while the soft-max is evaluated
+
+  stage(vbase, 0);  // the first V tile travels while the soft-max is evaluated
   // per row: max, exp, sequential f32 sum (attention.rs:28-38), divide, f16
-  for (int row = warp; row < rows; row += 8) {
-    const int Tr = t_first + row / group + 1;
-    float* e = sc + (size_t)row * cs;
+  for (int row = warp; row < rows; row += 4) {
+    const int Tr = (r0 + row) / group + 1;
+    float* e = reinterpret_cast<float*>(sc + row * cs);
     float mx = -INFINITY;
     for (int t = lane; t < Tr; t += 32) mx = fmaxf(mx, e[t]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+#pragma unroll 2
     for (int t = lane; t < Tr; t += 32) e[t] = exp_cr(__fsub_rn(e[t], mx));
-    __syncwarp();
-    float sum = 0.0f;
-    if (lane == 0) {
-      for (int t = 0; t < Tr; t++) sum = __fadd_rn(sum, e[t]);
+  }
+  __syncwarp();
+  float sum = 0.0f;   // lane i: the warp's row i
+  if (warp + 4 * lane < rows) {
+    const int row = warp + 4 * lane, Tr = (r0 + row) / group + 1;
+    const float* e = reinterpret_cast<const float*>(sc + row * cs);
+    int t = 0;
+#pragma unroll 4
+    for (; t + 4 <= Tr; t += 4) {
+      const float4 v = *reinterpret_cast<const float4*>(e + t);
+      sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, v.x), v.y), v.z), v.w);
     }
-    sum = __shfl_sync(0xffffffffu, sum, 0);
-    uint16_t* pr = p16 + (size_t)row * cs;
+    for (; t < Tr; t++) sum = __fadd_rn(sum, e[t]);
+  }
+  for (int row = warp, i = 0; row < rows; row += 4, i++) {
+    const int Tr = (r0 + row) / group + 1;
+    const float s = __shfl_sync(0xffffffffu, sum, i);
+    int* e = sc + row * cs;
     for (int t = lane; t < Tr; t += 32) {
-      float pv = e[t];
-      if (sum > 0.0f) pv = __fdiv_rn(pv, sum);
-      pr[t] = f32_to_f16_bits(pv);
+      float pv = __int_as_float(e[t]);
+      if (s > 0.0f) pv = __fdiv_rn(pv, s);
+      e[t] = f32_hi_large(f16_bits_to_f32(f32_to_f16_bits(pv)));
     }
   }
-  __syncthreads();
-  // out[row][d] = f32(sum_f64 over t ascending of v[t][d] * p[row][t]); thread -> (row, d) pairs, HD consecutive
-  // threads share a row so that p is a broadcast and v a conflict-free row read
-  constexpr int MAXO = 16;  // outputs per thread: QT * group * HD <= 256 * MAXO
-  double accv[MAXO];
+
+  // out[row][d] = f32(sum_f64 over t ascending of v[t][d] * p[row][t]): MMAs over the positions that every row sees (a
+  // multiple of four), the few after them one by one for the rows that see them
+  const int t_all = (r0 / group + 1) & ~3;
+  double acc[NT][2];
 #pragma unroll
-  for (int u = 0; u < MAXO; u++) accv[u] = 0.0;
-  const int n_out = rows * HD;
+  for (int n = 0; n < NT; n++) acc[n][0] = acc[n][1] = 0.0;
+  const int d0 = warp * (HD / 4);
+  const int* prow = sc + min(r, rows - 1) * cs;
   for (int tile = 0; tile < n_tiles; tile++) {
-    if (tile + 1 < n_tiles) stage(vbase, tile + 1, (tile + 1) & 1);
-    if (tile + 1 < n_tiles) cp_async_wait<1>(); else cp_async_wait<0>();
-    __syncthreads();
-    const uint16_t* vt = reinterpret_cast<const uint16_t*>(tiles + (size_t)(tile & 1) * tile_bytes);
-    const int t0 = tile * PF_TILE, nt = min(PF_TILE, T - t0);
+    if (tile + 1 < n_tiles) stage(vbase, tile + 1);
+    arrived(tile + 1 < n_tiles);
+    const int16_t* vt = kv + (tile & 1) * TILE + d0;
+    const int t0 = tile * PF_TILE, full = min(PF_TILE, t_all - t0), nt = min(PF_TILE, T - t0);
+#pragma unroll 4
+    for (int t = 0; t < full; t += 4) {
+      const double p = __hiloint2double(prow[t0 + t + c], 0);
 #pragma unroll
-    for (int u = 0; u < MAXO; u++) {
-      const int o = tid + u * 256;
-      if (o < n_out) {
-        const int row = o / HD, dd = o % HD;
-        const int lim = min(nt, t_first + row / group + 1 - t0);  // positions of this tile the row may see
-        const uint16_t* pr = p16 + (size_t)row * cs + t0;
-        double s = accv[u];
-        for (int tl = 0; tl < lim; tl++)
-          s += (double)__fmul_rn(f16_bits_to_f32(vt[(size_t)tl * HD + dd]), f16_bits_to_f32(pr[tl]));
-        accv[u] = s;
+      for (int n = 0; n < NT; n++) mma_f64(acc[n], p, f16_small_f64(vt[(t + c) * STRIDE + 8 * n + r]));
+    }
+    for (int t = max(full, 0); t < nt && t0 + t <= pos; t++) {
+      const double p = __hiloint2double(prow[t0 + t], 0);
+#pragma unroll
+      for (int n = 0; n < NT; n++) {
+        const uint32_t v2 = *reinterpret_cast<const uint32_t*>(vt + t * STRIDE + 8 * n + 2 * c);
+        acc[n][0] = __fma_rn(f16_small_f64((int16_t)(v2 & 0xffffu)), p, acc[n][0]);
+        acc[n][1] = __fma_rn(f16_small_f64((int16_t)(v2 >> 16)), p, acc[n][1]);
       }
     }
     __syncthreads();
   }
+  if (r < rows) {
+    float* o = attn_out + row_off + d0 + 2 * c;
 #pragma unroll
-  for (int u = 0; u < MAXO; u++) {
-    const int o = tid + u * 256;
-    if (o < n_out) {
-      const int row = o / HD, dd = o % HD;
-      const int qp = row / group, g = row % group;
-      attn_out[(bl * P + t_first + qp) * nq + (kvh * group + g) * HD + dd] = (float)accv[u];
-    }
+    for (int n = 0; n < NT; n++) *reinterpret_cast<float2*>(o + 8 * n) = make_float2((float)acc[n][0], (float)acc[n][1]);
   }
 }
 
@@ -239,29 +276,23 @@ __global__ void set_step_kernel(int* d_step, int value) {
   *d_step = value;
 }
 
-size_t prefill_attention_smem(int QT, int group, size_t T, size_t hd) {
-  const size_t cs = (T + 7) & ~(size_t)7, rows = (size_t)QT * group;
-  return rows * cs * 4 + rows * cs * 2 + rows * (hd + 2) * 2 + 16 + 2 * (size_t)PF_TILE * hd * 2;
+size_t prefill_attention_smem(int rows, size_t P, size_t hd) {
+  const size_t cs = (P + PF_TILE - 1) / PF_TILE * PF_TILE + 4;
+  return 2 * PF_TILE * (hd + 8) * 2 + rows * cs * 4;
 }
 
 }  // namespace
 
-// Largest number of query positions per CTA (a power of two up to 16) whose score rows fit in shared memory and
-// whose outputs fit the per-thread accumulators; 0 when even one position does not fit.
-int prefill_attention_qt(const rmi_ctx* ctx, const decode_dims& d, size_t P) {
-  const int group = (int)(d.n_head / d.n_head_kv);
-  // first choice: three CTAs per SM (their work grows with the query position, more CTAs even it out)
-  for (size_t limit : {(size_t)74 * 1024, ctx->smem_optin}) {
-    for (int qt = 16; qt >= 1; qt >>= 1) {
-      if ((size_t)qt * group * d.hd > 256 * 16) continue;
-      if (prefill_attention_smem(qt, group, P, d.hd) <= limit) return qt;
-    }
-  }
+// Query rows per CTA: the eight of an MMA row tile, fewer only where the scores of a long prompt leave no room.  0: none.
+// Sixteen rows (two row tiles share the conversion of K and V) are no faster: half as many CTAs even out less well.
+int prefill_attention_rows(const rmi_ctx* ctx, const decode_dims& d, size_t P) {
+  for (int rows = 8; rows >= 1; rows >>= 1)
+    if (prefill_attention_smem(rows, P, d.hd) <= ctx->smem_optin) return rows;
   return 0;
 }
 
 bool prefill_supported(const rmi_ctx* ctx, const decode_dims& d, size_t P) {
-  return (d.hd == 128 || d.hd == 64 || d.hd == 32) && d.n_head % d.n_head_kv == 0 && prefill_attention_qt(ctx, d, P) > 0;
+  return (d.hd == 128 || d.hd == 64 || d.hd == 32) && d.n_head % d.n_head_kv == 0 && prefill_attention_rows(ctx, d, P) > 0;
 }
 
 int32_t launch_embed_rows(rmi_ctx* ctx, const rmi_weight* emb, const uint32_t* prompts, size_t n_prompt, size_t P, size_t b0,
@@ -285,21 +316,18 @@ int32_t launch_qk_norm_rope_kv_rows(rmi_ctx* ctx, const decode_dims& d, const fl
 
 int32_t launch_attention_prefill(rmi_ctx* ctx, const decode_dims& d, const uint16_t* q16, const uint16_t* k_cache,
                                  const uint16_t* v_cache, size_t layer, size_t P, size_t b0, size_t n_seq, float* attn_out) {
-  const int qt = prefill_attention_qt(ctx, d, P);
-  RMI_REQUIRE(qt > 0, RMI_ERR_UNSUPPORTED, "prompt of %zu positions does not fit the prefill attention kernel", P);
-  const int group = (int)(d.n_head / d.n_head_kv);
-  const size_t smem = prefill_attention_smem(qt, group, P, d.hd);
-  void (*kern)(const uint16_t*, const uint16_t*, const uint16_t*, size_t, size_t, size_t, size_t, size_t, size_t, size_t, int,
-               float*) = d.hd == 128 ? attention_prefill_kernel<128>
-                                     : (d.hd == 64 ? attention_prefill_kernel<64> : attention_prefill_kernel<32>);
+  const int rows = prefill_attention_rows(ctx, d, P);
+  RMI_REQUIRE(rows > 0, RMI_ERR_UNSUPPORTED, "prompt of %zu positions does not fit the prefill attention kernel", P);
+  const size_t group = d.n_head / d.n_head_kv, smem = prefill_attention_smem(rows, P, d.hd);
+  auto kern = d.hd == 128 ? attention_prefill_kernel<128> : (d.hd == 64 ? attention_prefill_kernel<64> : attention_prefill_kernel<32>);
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
     (void)cudaGetLastError();
     rmi_set_error("prefill attention needs %zu B of shared memory", smem);
     return RMI_ERR_UNSUPPORTED;
   }
-  dim3 grid((unsigned)((P + qt - 1) / qt), (unsigned)d.n_head_kv, (unsigned)n_seq);
-  return rmi_run(ctx, "attention_prefill", kern, grid, dim3(256), smem, q16, k_cache, v_cache, d.n_head, d.n_head_kv, layer, d.n_layer,
-                 d.capacity, P, b0, qt, attn_out);
+  const size_t grid = (P * group + rows - 1) / rows * d.n_head_kv * n_seq;
+  return rmi_run(ctx, "attention_prefill", kern, dim3((unsigned)grid), dim3(PF_THREADS), smem, q16, k_cache, v_cache, d.n_head, d.n_head_kv, layer,
+                 d.n_layer, d.capacity, P, b0, n_seq, rows, attn_out);
 }
 
 int32_t launch_set_step(rmi_ctx* ctx, int* d_step, int value) {

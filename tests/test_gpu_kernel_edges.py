@@ -66,3 +66,24 @@ def test_kernel_trait_forward_batched(rmi, ctx, kind, m, n, k):
         else:
             ref = orc.q6k_forward_prepared(wb, x[t], k, n)
         assert np.array_equal(bits(got[t]), bits(ref)), t
+
+
+# every head size, one to eight query heads per kv head, prompts that end on and beside the edges of row and position tiles
+@pytest.mark.parametrize("head_dim,n_head,n_head_kv,positions", [(32, 8, 1, 16), (64, 4, 2, 64), (128, 4, 4, 65), (128, 2, 1, 131)])
+def test_prefill_attention_rows_and_heads(rmi, ctx, tmp_path, head_dim, n_head, n_head_kv, positions):
+    from tests.synth_model import tiny_cfg
+    cfg = tiny_cfg(head_dim=head_dim, n_head=n_head, n_head_kv=n_head_kv)
+    path = str(tmp_path / "m.gguf")
+    rmi.synth.write_qwen3_gguf(path, cfg, rmi.synth.qwen3_tensors(cfg, 3))
+    model = rmi.Qwen3Model.from_file(path)
+    prompts = np.stack([rmi.synth.prompt_tokens(cfg["vocab"], positions + 1, seed=b) for b in range(2)])
+    s = rmi.Qwen3Session(model, positions + 8, batch=2)
+    got = []
+    for mode in (rmi.PREFILL_TOKEN_LOOP, rmi.PREFILL_BATCHED):
+        s.set_prefill(mode)
+        tok = s.generate(prompts, 4)
+        got.append((tok, bits(s.hidden()), bits(s.logits())))
+    for loop, batched in zip(*got):
+        assert np.array_equal(loop, batched)
+    s.free()
+    model.free()
