@@ -27,12 +27,13 @@ extern "C" int32_t rmi_quantize_q8_k(rmi_ctx* ctx, const float* x, size_t m, siz
   return RMI_OK;
 }
 
-// Quantize to Q8_K, then Q4_K x Q8_K; caller holds ctx->mu.  The tensor-core kernel takes over where the weights are no
-// longer what a call waits for; it exists for the AVX2 order only.
-static constexpr size_t Q4K_MMA_MIN_M = 16;
+// Quantize to Q8_K, then Q4_K x Q8_K; caller holds ctx->mu.  The tensor-core kernel exists for the AVX2 order only; up to 16
+// rows cost it what one does, so it takes over from the passes of the streaming kernels at three (4096 x 4096: 1, 2, 4, 8
+// rows streamed 10, 10, 16, 20 us; on the tensor cores 10).
+static constexpr size_t Q4K_Q8K_MMA_MIN_M = 3;
 
 static int32_t q4k_q8k_device(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, float* out, size_t row_begin, size_t row_end) {
-  if (m >= Q4K_MMA_MIN_M && ctx->sem == RMI_SEM_AVX2) {
+  if (m >= Q4K_Q8K_MMA_MIN_M && ctx->sem == RMI_SEM_AVX2 && q4k_mma_prepare(ctx, w, false)) {
     uint8_t* xrec;
     RMI_TRY(rmi_scratch(ctx, 0, q4k_mma_x_bytes(w, m, false), (void**)&xrec));
     return launch_q4k_q8k_mma(ctx, w, x, m, xrec, out, row_begin, row_end);
@@ -76,8 +77,13 @@ extern "C" int32_t rmi_matmul_q4_k_q8k_dev(rmi_ctx* ctx, const rmi_weight* w, co
   return q4k_q8k_device(ctx, w, x, m, output, 0, w->n_rows);
 }
 
+// The time of the tensor-core kernel for few rows is that of one CTA walking K, whatever the number of weight rows that the
+// SMs hold at once: 23 us for K = 4096 with 4096 or 11008 rows, where 8 activation rows take the streaming kernel 18 and
+// 47 us, 12 take it 33 and 73.
+static bool q4k_dequant_on_mma(const rmi_weight* w, size_t m) { return m >= 9 || (m >= 5 && w->n_rows >= 8192); }
+
 static int32_t q4k_dequant_device(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, float* out) {
-  if (m < Q4K_MMA_MIN_M) return launch_q4k_dequant_matmul(ctx, w, x, m, out);
+  if (!q4k_dequant_on_mma(w, m) || !q4k_mma_prepare(ctx, w, true)) return launch_q4k_dequant_matmul(ctx, w, x, m, out);
   uint8_t* xrec;
   RMI_TRY(rmi_scratch(ctx, 0, q4k_mma_x_bytes(w, m, true), (void**)&xrec));
   return launch_q4k_dequant_mma(ctx, w, x, m, xrec, out);

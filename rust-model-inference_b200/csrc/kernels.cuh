@@ -89,6 +89,7 @@ int32_t launch_q4k_q8k_matmul(rmi_ctx* ctx, const rmi_weight* w, const float* d8
 int32_t launch_q4k_dequant_matmul(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, float* out);
 int32_t launch_q4k_dequantize(rmi_ctx* ctx, const rmi_weight* w, float* out);
 // q4k_mma.cu (tensor cores, many activation rows): f32 rows in, scratch of q4k_mma_x_bytes for their records
+bool q4k_mma_prepare(rmi_ctx* ctx, const rmi_weight* w, bool dequant);
 size_t q4k_mma_x_bytes(const rmi_weight* w, size_t m, bool dequant);
 int32_t launch_q4k_q8k_mma(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, uint8_t* xrec, float* out, size_t row_begin,
                            size_t row_end);

@@ -232,159 +232,6 @@ __global__ void q4k_q8k_matmul_kernel(const uint8_t* __restrict__ w, size_t nb, 
   }
 }
 
-// Q4_K x Q8_K for many activation rows: a tiled kernel instead of one pass over the weights per group of rows.
-// CTA tile: 32 weight rows x 16 activation rows, one super-block (256 values) per step, two shared-memory stages
-// filled with cp.async.  Thread = (4 weight rows 4tn..4tn+3 x 4 activation rows tm, tm+4, tm+8, tm+12, AVX2 lane L): for every pair of its
-// tile it forms lane L's integer sum  v_L = sum_j sc[2j] * dot4(lo nibbles) + sc[2j+1] * dot4(hi nibbles)  over
-// the four 64-value groups (exact; mod.rs:759-783) and accumulates acc_L = fma(d_w * d_x, f32(v_L), acc_L) over
-// the super-blocks in order, plus the mins term of lane L & 3 (mod.rs:749-756) -- the same per-lane chains as the
-// row kernel above, so the f32 result is bit-identical; the eight lanes of a pair sit in eight neighbouring
-// threads and are combined at the end exactly as hsum_ps does (dot.rs:447-456).
-constexpr int Q4T_TN = 32, Q4T_TM = 16;
-// activation rows padded to 288 B (16-byte aligned for cp.async; 72 words, so the four row groups of a warp, one row
-// apart, fall into different banks)
-constexpr int Q4T_XSTRIDE = 288;
-
-struct q4t_stage {
-  uint8_t wq[Q4T_TN][144];            // raw super-blocks of the weight rows
-  int8_t xq[Q4T_TM][Q4T_XSTRIDE];     // quantized activations
-  int16_t xb[Q4T_TM][16];             // bsums
-  float xd[Q4T_TM];                   // d
-};
-
-__global__ void __launch_bounds__(256)
-    q4k_q8k_tiled_kernel(const uint8_t* __restrict__ w, size_t nb, size_t n_rows, const float* __restrict__ d8,
-                         const int8_t* __restrict__ q8, const int16_t* __restrict__ bs, size_t m_rows,
-                         float* __restrict__ out, size_t row_begin, size_t row_end) {
-  __shared__ __align__(16) q4t_stage stg[2];
-  __shared__ int s_sc[2][Q4T_TN][8], s_mn[2][Q4T_TN][8];   // 6-bit scales and mins, decoded once per (row, super-block)
-  __shared__ float s_wd[2][Q4T_TN][2];                     // d, dmin
-  __shared__ int s_xs[2][Q4T_TM][8];                       // pairwise bsum sums (i16 wrap): [tt][0], [tt][1]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int L = lane & 7, tm = lane >> 3, tn = warp;       // 4 activation-row tiles per warp share the weight tile
-  pdl_wait();
-  pdl_launch_dependents();
-  const size_t n0 = row_begin + (size_t)blockIdx.x * Q4T_TN, m0 = (size_t)blockIdx.y * Q4T_TM;
-
-  auto load_stage = [&](int st, size_t i) {
-    // weights: 32 rows x 144 B = 288 16-byte pieces; activations: 16 rows x 256 B = 256 pieces; bsums 16 x 32 B
-    for (int p = tid; p < Q4T_TN * 9; p += 256) {
-      const int r = p / 9, c = p % 9;
-      const size_t row = n0 + r < row_end ? n0 + r : row_end - 1;  // rows past the range repeat the last one (never stored)
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(&stg[st].wq[r][c * 16])),
-                   "l"(w + (row * nb + i) * 144 + c * 16)
-                   : "memory");
-    }
-    {
-      const int r = tid / 16, c = tid % 16;
-      const size_t t = m0 + r < m_rows ? m0 + r : m_rows - 1;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(&stg[st].xq[r][c * 16])),
-                   "l"(q8 + (t * nb + i) * 256 + c * 16)
-                   : "memory");
-    }
-    if (tid < Q4T_TM * 2) {
-      const int r = tid / 2, c = tid % 2;
-      const size_t t = m0 + r < m_rows ? m0 + r : m_rows - 1;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(&stg[st].xb[r][c * 8])),
-                   "l"(bs + (t * nb + i) * 16 + c * 8)
-                   : "memory");
-    }
-    if (tid < Q4T_TM) {
-      const size_t t = m0 + tid < m_rows ? m0 + tid : m_rows - 1;
-      stg[st].xd[tid] = d8[t * nb + i];
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  auto decode_stage = [&](int st) {
-    if (tid < Q4T_TN * 8) {
-      const int r = tid >> 3, jj = tid & 7;
-      const uint32_t* h = reinterpret_cast<const uint32_t*>(stg[st].wq[r]);
-      int sc, mn;
-      scale_min_w(h[1], h[2], h[3], jj, &sc, &mn);
-      s_sc[st][r][jj] = sc;
-      s_mn[st][r][jj] = mn;
-      if (jj == 0) {
-        s_wd[st][r][0] = f16_bits_to_f32((uint16_t)(h[0] & 0xffffu));
-        s_wd[st][r][1] = f16_bits_to_f32((uint16_t)(h[0] >> 16));
-      }
-    }
-    if (tid < Q4T_TM * 8) {
-      const int r = tid >> 3, k = tid & 7;   // k = 2 * tt + which
-      const int16_t* b = stg[st].xb[r] + 2 * k;
-      s_xs[st][r][k] = (int)(int16_t)(b[0] + b[1]);  // hadd_epi16 wraps to i16 (mod.rs:749-752)
-    }
-  };
-
-  float acc[4][4], accm[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int b = 0; b < 4; b++) acc[a][b] = accm[a][b] = 0.0f;
-
-  load_stage(0, 0);
-  for (size_t i = 0; i < nb; i++) {
-    const int st = (int)(i & 1);
-    if (i + 1 < nb) load_stage(st ^ 1, i + 1);
-    if (i + 1 < nb) asm volatile("cp.async.wait_group 1;" ::: "memory");
-    else asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-    decode_stage(st);
-    __syncthreads();
-    const q4t_stage& S = stg[st];
-    int v[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-      for (int b = 0; b < 4; b++) v[a][b] = 0;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      int xlo[4], xhi[4];
-#pragma unroll
-      for (int b = 0; b < 4; b++) {
-        xlo[b] = *reinterpret_cast<const int*>(&S.xq[tm + 4 * b][64 * j + 4 * L]);
-        xhi[b] = *reinterpret_cast<const int*>(&S.xq[tm + 4 * b][64 * j + 32 + 4 * L]);
-      }
-#pragma unroll
-      for (int a = 0; a < 4; a++) {
-        const int r = tn * 4 + a;
-        const uint32_t wq = *reinterpret_cast<const uint32_t*>(&S.wq[r][16 + 32 * j + 4 * L]);
-        const int sc0 = s_sc[st][r][2 * j], sc1 = s_sc[st][r][2 * j + 1];
-        const int wlo = (int)(wq & 0x0F0F0F0Fu), whi = (int)((wq >> 4) & 0x0F0F0F0Fu);
-#pragma unroll
-        for (int b = 0; b < 4; b++) v[a][b] += sc0 * dp4a_s8(wlo, xlo[b], 0) + sc1 * dp4a_s8(whi, xhi[b], 0);
-      }
-    }
-    const int tt = L & 3;
-#pragma unroll
-    for (int a = 0; a < 4; a++) {
-      const int r = tn * 4 + a;
-      const float dw = s_wd[st][r][0], dminw = s_wd[st][r][1];
-      const int ma = s_mn[st][r][2 * tt], mb = s_mn[st][r][2 * tt + 1];
-#pragma unroll
-      for (int b = 0; b < 4; b++) {
-        const int t = tm + 4 * b;
-        const float dq = S.xd[t];
-        acc[a][b] = __fmaf_rn(__fmul_rn(dw, dq), (float)v[a][b], acc[a][b]);
-        accm[a][b] = __fmaf_rn(__fmul_rn(-dminw, dq), (float)(ma * s_xs[st][t][2 * tt] + mb * s_xs[st][t][2 * tt + 1]), accm[a][b]);
-      }
-    }
-    __syncthreads();  // the stage is refilled by the loads issued in the next iteration
-  }
-#pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int b = 0; b < 4; b++) {
-      // hsum_ps over lanes L = 0..7 (dot.rs:447-456), mins: (m0+m2)+(m1+m3) (mod.rs:792-794)
-      const float s1 = __fadd_rn(__shfl_xor_sync(0xffffffffu, acc[a][b], 4), acc[a][b]);
-      const float u = __fadd_rn(s1, __shfl_xor_sync(0xffffffffu, s1, 1));
-      const float main_val = __fadd_rn(u, __shfl_xor_sync(0xffffffffu, u, 2));
-      const float m02 = __fadd_rn(accm[a][b], __shfl_xor_sync(0xffffffffu, accm[a][b], 2));
-      const float min_val = __fadd_rn(m02, __shfl_xor_sync(0xffffffffu, m02, 1));
-      const size_t row = n0 + tn * 4 + a, t = m0 + tm + 4 * b;
-      if (L == 0 && row < row_end && t < m_rows) out[t * n_rows + row] = __fadd_rn(main_val, min_val);
-    }
-}
-
 // The sixteen 6-bit fields of a super-block header (mod.rs:25-33) unpacked four at a time on whole words:
 // h1..h3 are the 12 scale bytes; the results hold sc[0..3], sc[4..7], mn[0..3], mn[4..7] as bytes.
 struct q4k_fields {
@@ -822,137 +669,6 @@ __global__ void q4k_dequant_matmul_kernel(const uint8_t* __restrict__ w, size_t 
     }
 }
 
-// forward_dequant for many activation rows (compute-bound in f32): a register-tiled f32 GEMM whose weight tile
-// is decoded from the Q4_K bytes on the way into shared memory (same w = (d*sc)*q - dmin*m arithmetic as above,
-// mod.rs:471-486).  CTA tile 128 weight rows x 64 activation rows, K chunks of 32 values (one half of a 64-value
-// group: the low or the high nibbles of 32 quant bytes, one 6-bit scale/min pair), 256 threads with 8 x 4
-// accumulators each, two shared-memory stages.
-constexpr int Q4G_BN = 128, Q4G_BM = 64, Q4G_BK = 32, Q4G_PAD = 4;
-// Two groups of 256 threads share a tile and take alternate K chunks (each with its own pair of shared-memory
-// stages and its own named barrier), so that a CTA brings 16 warps to an SM: a 4096 x 4096 weight with 256
-// activation rows is only 128 tiles, and 8 warps per SM leave the FMA pipe idle most of the time.  The two
-// partial tiles are added at the end (group 0 + group 1); forward_dequant carries a tolerance, not an order.
-constexpr int Q4G_KGROUPS = 2;
-constexpr size_t Q4G_GROUP_SMEM = 2 * Q4G_BK * (Q4G_BN + Q4G_PAD + Q4G_BM + Q4G_PAD) * 4;
-
-__global__ void __launch_bounds__(256 * Q4G_KGROUPS)
-    q4k_dequant_gemm_kernel(const uint8_t* __restrict__ w, size_t nb, size_t n_rows, const float* __restrict__ x,
-                            size_t m_rows, float* __restrict__ out) {
-  extern __shared__ __align__(16) uint8_t q4g_smem[];
-  pdl_wait();
-  pdl_launch_dependents();
-  const int kg = threadIdx.x >> 8, tid = threadIdx.x & 255;
-  uint8_t* gsm = q4g_smem + (size_t)kg * Q4G_GROUP_SMEM;
-  float (*Ws)[Q4G_BK][Q4G_BN + Q4G_PAD] = reinterpret_cast<float (*)[Q4G_BK][Q4G_BN + Q4G_PAD]>(gsm);
-  float (*Xs)[Q4G_BK][Q4G_BM + Q4G_PAD] =
-      reinterpret_cast<float (*)[Q4G_BK][Q4G_BM + Q4G_PAD]>(gsm + 2 * Q4G_BK * (Q4G_BN + Q4G_PAD) * 4);
-  const size_t n0 = (size_t)blockIdx.x * Q4G_BN, m0 = (size_t)blockIdx.y * Q4G_BM;
-  const size_t K = nb * 256;
-  const int n_chunks = (int)(nb * 8);   // a multiple of 8: both groups walk the same number of chunks
-  auto group_sync = [&]() { asm volatile("bar.sync %0, 256;" ::"r"(1 + kg) : "memory"); };
-  // loader roles: weights - thread (row tid/2, 16 of the chunk's 32 values); activations - thread (row tid/4, 8 values)
-  const int wr = tid >> 1, wh = tid & 1;
-  const int xr = tid >> 2, xq = tid & 3;
-  const bool w_ok = n0 + wr < n_rows, x_ok = m0 + xr < m_rows;
-  const uint8_t* wrow = w + (n0 + wr) * nb * 144;
-  const float* xrow = x + (m0 + xr) * K;
-  // compute roles: tx = weight rows 4tx..4tx+3 and 64+4tx..64+4tx+3 (the sixteen tx of a warp read 256 contiguous
-  // bytes per load: no bank conflict), ty = 4 consecutive activation rows
-  const int tx = tid & 15, ty = tid >> 4;
-  float acc[4][8];
-#pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int b = 0; b < 8; b++) acc[a][b] = 0.0f;
-
-  uint4 qv = make_uint4(0u, 0u, 0u, 0u), hv = make_uint4(0u, 0u, 0u, 0u);
-  float4 xa = make_float4(0.f, 0.f, 0.f, 0.f), xb = xa;
-  auto fetch = [&](int c) {
-    const int sb = c >> 3, cc = c & 7, grp = cc >> 1;
-    if (w_ok) {
-      const uint8_t* blk = wrow + (size_t)sb * 144;
-      hv = __ldg(reinterpret_cast<const uint4*>(blk));
-      qv = __ldg(reinterpret_cast<const uint4*>(blk + 16 + 32 * grp + 16 * wh));
-    }
-    if (x_ok) {
-      const float* xp = xrow + (size_t)c * Q4G_BK + xq * 8;
-      xa = __ldg(reinterpret_cast<const float4*>(xp));
-      xb = __ldg(reinterpret_cast<const float4*>(xp + 4));
-    }
-  };
-  auto stash = [&](int c, int st) {
-    const int cc = c & 7, hi = cc & 1;
-    int sc, mn;
-    scale_min_w(hv.y, hv.z, hv.w, cc, &sc, &mn);
-    const float d1 = __fmul_rn(f16_bits_to_f32((uint16_t)(hv.x & 0xffffu)), (float)sc);
-    const float m1 = __fmul_rn(f16_bits_to_f32((uint16_t)(hv.x >> 16)), (float)mn);
-    const float c1 = -__fmul_rn(d1, 8388608.0f);
-    const uint32_t q[4] = {qv.x, qv.y, qv.z, qv.w};
-#pragma unroll
-    for (int v4 = 0; v4 < 4; v4++) {
-      const uint32_t nib = hi ? (q[v4] >> 4) & 0x0F0F0F0Fu : q[v4] & 0x0F0F0F0Fu;
-#pragma unroll
-      for (int v = 0; v < 4; v++)   // (d*sc)*q as fma(d*sc, 2^23 + q, -(d*sc)*2^23): exact product, one rounding
-        Ws[st][wh * 16 + 4 * v4 + v][wr] = w_ok ? __fsub_rn(__fmaf_rn(d1, byte_plus_2p23(nib, v), c1), m1) : 0.0f;
-    }
-    const float xv[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
-#pragma unroll
-    for (int v = 0; v < 8; v++) Xs[st][xq * 8 + v][xr] = x_ok ? xv[v] : 0.0f;
-  };
-
-  fetch(kg);
-  stash(kg, 0);
-  group_sync();
-  for (int c = kg, it = 0; c < n_chunks; c += Q4G_KGROUPS, it++) {
-    const int st = it & 1;
-    if (c + Q4G_KGROUPS < n_chunks) fetch(c + Q4G_KGROUPS);
-#pragma unroll
-    for (int k = 0; k < Q4G_BK; k++) {
-      const float4 a0 = *reinterpret_cast<const float4*>(&Ws[st][k][tx * 4]);
-      const float4 a1 = *reinterpret_cast<const float4*>(&Ws[st][k][64 + tx * 4]);
-      const float4 b0 = *reinterpret_cast<const float4*>(&Xs[st][k][ty * 4]);
-      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      const float bv[4] = {b0.x, b0.y, b0.z, b0.w};
-#pragma unroll
-      for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 8; b++) acc[a][b] = __fmaf_rn(av[b], bv[a], acc[a][b]);
-    }
-    if (c + Q4G_KGROUPS < n_chunks) stash(c + Q4G_KGROUPS, st ^ 1);
-    group_sync();
-  }
-  // group 1 hands its partial tile over through its own (now idle) stages: [32 values][256 threads]
-  float* hand = reinterpret_cast<float*>(q4g_smem + Q4G_GROUP_SMEM);
-  if (kg == 1) {
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-      for (int b = 0; b < 8; b++) hand[(a * 8 + b) * 256 + tid] = acc[a][b];
-  }
-  __syncthreads();
-  if (kg != 0) return;
-#pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int b = 0; b < 8; b++) acc[a][b] = __fadd_rn(acc[a][b], hand[(a * 8 + b) * 256 + tid]);
-#pragma unroll
-  for (int a = 0; a < 4; a++) {
-    const size_t mrow = m0 + ty * 4 + a;
-    if (mrow >= m_rows) continue;
-    float* o = out + mrow * n_rows + n0 + tx * 4;   // columns 4tx..4tx+3, then 64 further on
-    if (n0 + 64 + tx * 4 + 4 <= n_rows && (n_rows & 3) == 0) {
-      *reinterpret_cast<float4*>(o) = make_float4(acc[a][0], acc[a][1], acc[a][2], acc[a][3]);
-      *reinterpret_cast<float4*>(o + 64) = make_float4(acc[a][4], acc[a][5], acc[a][6], acc[a][7]);
-    } else {
-#pragma unroll
-      for (int b = 0; b < 8; b++) {
-        const size_t col = n0 + tx * 4 + (b < 4 ? b : 60 + b);
-        if (col < n_rows) out[mrow * n_rows + col] = acc[a][b];
-      }
-    }
-  }
-}
-
 __global__ void q4k_dequantize_kernel(const uint8_t* __restrict__ w, size_t n_superblocks, float* __restrict__ out) {
   const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
   const int lane = threadIdx.x & 31;
@@ -1049,12 +765,6 @@ int32_t launch_q4k_q8k_matmul(rmi_ctx* ctx, const rmi_weight* w, const float* d8
                               const int16_t* bsums, size_t m, float* out, size_t row_begin, size_t row_end) {
   if (m == 0 || row_begin >= row_end) return RMI_OK;
   const size_t nb = w->n_in / 256;
-  if (m >= 32 && ctx->sem != RMI_SEM_SCALAR) {
-    // many rows: tiled kernel, every weight super-block is fetched once per 16 activation rows
-    dim3 grid((unsigned)((row_end - row_begin + Q4T_TN - 1) / Q4T_TN), (unsigned)((m + Q4T_TM - 1) / Q4T_TM));
-    return rmi_run(ctx, "q4k_q8k_tiled", q4k_q8k_tiled_kernel, grid, dim3(256), 0, w->d_raw, nb, w->n_rows, d8, qs, bsums, m, out,
-                   row_begin, row_end);
-  }
   if (ctx->sem != RMI_SEM_SCALAR) {
     // few rows: groups of 8 / 4 activation rows through the streaming kernel (16-row tiles, whole rows per warp),
     // groups of 2 / 1 through the split-K kernel (4-row tiles, the super-blocks of a row over four warps)
@@ -1093,15 +803,6 @@ int32_t launch_q4k_q8k_matmul(rmi_ctx* ctx, const rmi_weight* w, const float* d8
 int32_t launch_q4k_dequant_matmul(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, float* out) {
   if (m == 0 || w->n_rows == 0) return RMI_OK;
   const size_t nb = w->n_in / 256;
-  if (m >= 32) {  // compute-bound: tiled f32 GEMM with on-the-fly decode
-    dim3 g2((unsigned)((w->n_rows + Q4G_BN - 1) / Q4G_BN), (unsigned)((m + Q4G_BM - 1) / Q4G_BM));
-    constexpr size_t smem = Q4G_KGROUPS * Q4G_GROUP_SMEM;
-    if (cudaFuncSetAttribute(q4k_dequant_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-      rmi_set_error("cudaFuncSetAttribute(%zu B shared) failed", smem);
-      return RMI_ERR_CUDA;
-    }
-    return rmi_run(ctx, "q4k_dequant_gemm", q4k_dequant_gemm_kernel, g2, dim3(256 * Q4G_KGROUPS), smem, w->d_raw, nb, w->n_rows, x, m, out);
-  }
   size_t t = 0;
   while (t < m) {
     const size_t left = m - t;

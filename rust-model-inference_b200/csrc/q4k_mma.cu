@@ -1,22 +1,25 @@
 // Q4_K matmuls of many activation rows on the tensor cores: the dequantize-and-matmul path and the Q4_K x Q8_K path in
 // its exact AVX2 order.  Both use warp-level MMAs (m16n8k16, f32 results in the registers of the threads that scale
 // them): the results of two to six MMAs are scaled by per-block factors, so no accumulator could stay in tensor memory
-// for longer than that, and the MMA rate (8 cycles per 2048 products and SM sub-partition, measured) is what bounds both.
+// for longer than that.
 //
 //   Q4_K x Q8_K (src/ops/quant/mod.rs:701-799).  AVX2 lane L of a super-block sums sc * q * x over 32 values in integers,
 //   then acc_L = fma(d_w * d_x, f32(sum), acc_L).  sc * q <= 945 and the bytes x are exact in f16, and a sum of 32 such
 //   products is below 2^22, so two m16n8k16 deliver f32(sum) exactly; the eight lanes are eight such pairs on the same
 //   operands' other words.  The mins' four chains (mod.rs:749-756) run beside them on exact f32 integers.
-//   CUDA cores (dp4a, 16 x 32 tiles): 33 TOPS on 11008 x 4096 with 200 rows; here see the table of the launcher.
+//   Bound: no single unit (per warp and super-block of 16 x 16 rows: MMAs 256 cycles of a sub-partition, shared-memory loads
+//   400 of the SM, about 400 instructions), at two warps per sub-partition.  11008 x 4096, 200 rows: 116 us (dp4a: 543).
 //
 //   Dequantize (mod.rs:471-486, tolerance 1e-4): w = (d*sc) * q - dmin*m, so the dot over a 32-block is
 //   (d*sc) * sum(q * x) - (dmin*m) * sum(x).  q is exact in bf16 and x is the exact sum of three bf16 values (8 + 8 + 8
 //   significant bits), so sum(q * x) is six m16n8k16 with f32 accumulation: no input is rounded.
+//   Bound: the MMA rate (8 cycles per 2048 products and sub-partition: 53 us) and the operand loads from shared memory, which
+//   take half as long with two weight tiles per warp.  4096 x 4096, 300 rows: 112 us (CUDA cores: 545).
 //
 // Weights are re-laid out once per path into records whose bytes are in operand-register order (a thread's share of a
-// fragment is one aligned piece), activations are written that way by their quantizer / splitter.  The records of four
-// weight tiles (64 rows) and of four activation groups (32 rows) lie together, K step after K step, so that a stage of a
-// CTA's ring is one bulk copy of either kind: every further copy costs the issuing warp a few hundred cycles, and with
+// fragment is one aligned piece), activations are written that way by their quantizer / splitter.  The records of the
+// weight tiles and of the activation groups of a CTA lie together, K step after K step, so that a stage of its ring is one
+// bulk copy of either kind: every further copy costs the issuing warp a few hundred cycles, and with
 // one copy per tile the kernels took the sum of their copy and arithmetic times.
 #include "common.cuh"
 #include "kernels.cuh"
@@ -51,37 +54,41 @@ struct q4k_params {
   rmi_dev_status* status;
 };
 
-constexpr int PACK = 4;   // weight tiles / activation groups whose records lie together
-__host__ __device__ constexpr size_t packed(size_t i, size_t steps, size_t step) {   // record index
-  return (i / PACK * steps + step) * PACK + i % PACK;
+// Weight tiles whose records lie together: those of a CTA.  Of activation groups it is the CTA's number of them, 1 or 2.
+constexpr int Q8K_W_PACK = 4, DEQ_W_PACK = 8, X_PACK_MAX = 2;
+__host__ __device__ constexpr size_t packed(int pack, size_t i, size_t steps, size_t step) {   // record index
+  return (i / pack * steps + step) * pack + i % pack;
 }
 
-// RT weight tiles (PACK of them) x TG activation groups (a divisor of PACK).
-template <int RT, int TG, int WREC, int XREC, int S>
+// RT weight tiles x TG activation groups, KC records of each per stage (several: a stage's barriers and copies take its
+// warps a few hundred cycles).
+template <int RT, int TG, int WREC, int XREC, int KC, int S>
 struct q4k_ring {
-  static_assert(RT == PACK && PACK % TG == 0 && S <= 7, "one copy per operand");
-  static constexpr int B0 = RT * WREC, STAGE = B0 + TG * XREC, SMEM = 128 + S * STAGE;
-  int tile, step;
+  static_assert(S <= 7, "barriers");
+  static constexpr int W_STEP = RT * WREC, X_STEP = TG * XREC;
+  static constexpr int B0 = KC * W_STEP, STAGE = B0 + KC * X_STEP, SMEM = 128 + S * STAGE;
+  int tile, chunk;   // the next item
+  __device__ __forceinline__ int blocks(const q4k_params& p) const { return min(KC, p.steps - chunk * KC); }
   __device__ __forceinline__ void copy_w(const q4k_params& p, uint32_t smem, int st) const {
-    const int tr = tile / p.tiles_t;
-    bulk_load(smem + 128 + st * STAGE, p.w + packed((size_t)p.rt0 + tr * RT, p.steps, step) * WREC, RT * WREC, smem + 8 * st);
+    const size_t tr = p.rt0 / RT + tile / p.tiles_t;
+    bulk_load(smem + 128 + st * STAGE, p.w + (tr * p.steps + chunk * KC) * W_STEP, blocks(p) * W_STEP, smem + 8 * st);
   }
   __device__ __forceinline__ void copy_x(const q4k_params& p, uint32_t smem, int st) const {
-    const int tt = tile % p.tiles_t;
-    bulk_load(smem + 128 + st * STAGE + B0, p.x + packed((size_t)tt * TG, p.steps, step) * XREC, TG * XREC, smem + 8 * st);
+    const size_t tt = tile % p.tiles_t;
+    bulk_load(smem + 128 + st * STAGE + B0, p.x + (tt * p.steps + chunk * KC) * X_STEP, blocks(p) * X_STEP, smem + 8 * st);
   }
   __device__ __forceinline__ void advance(const q4k_params& p) {
-    if (++step == p.steps) step = 0, tile += gridDim.x;
+    if (++chunk * KC >= p.steps) chunk = 0, tile += gridDim.x;
   }
-  // The first S records, by one thread; the weights' part travels before the wait on the preceding kernel, which writes
+  // The first S stages, by one thread; the weights' part travels before the wait on the preceding kernel, which writes
   // activations only.
   __device__ __forceinline__ void start(const q4k_params& p, uint32_t smem) {
     for (int pass = 0; pass < 2; pass++) {
       if (pass == 1) pdl_wait();
-      tile = blockIdx.x, step = 0;
+      tile = blockIdx.x, chunk = 0;
       for (int st = 0; st < S && tile < p.n_tiles; st++) {
         if (pass == 0) {
-          mbar_expect_tx(smem + 8 * st, STAGE);
+          mbar_expect_tx(smem + 8 * st, blocks(p) * (W_STEP + X_STEP));
           copy_w(p, smem, st);
         } else {
           copy_x(p, smem, st);
@@ -90,15 +97,14 @@ struct q4k_ring {
       }
     }
   }
-  __device__ __forceinline__ bool next(const q4k_params& p, uint32_t smem, int item, int* abort_flag) {
-    if (tile >= p.n_tiles) return true;
+  __device__ __forceinline__ void next(const q4k_params& p, uint32_t smem, int item, int* abort_flag) {
+    if (tile >= p.n_tiles) return;
     const int st = item % S;
-    if (!mbar_wait(smem + 64 + 8 * st, ((item / S) & 1) ^ 1, abort_flag, p.status, 15, item)) return false;
-    mbar_expect_tx(smem + 8 * st, STAGE);
+    if (!mbar_wait(smem + 64 + 8 * st, ((item / S) & 1) ^ 1, abort_flag, p.status, 15, item)) return;
+    mbar_expect_tx(smem + 8 * st, blocks(p) * (W_STEP + X_STEP));
     copy_w(p, smem, st);
     copy_x(p, smem, st);
     advance(p);
-    return true;
   }
 };
 
@@ -124,10 +130,11 @@ __device__ __forceinline__ uint32_t lop_or(uint32_t w, uint32_t mask, uint32_t b
 // ---------------------------------------------------------------- Q4_K x Q8_K
 
 // Warp tile: 16 weight rows x 8 NG activation rows.
-template <int NG, int NWR, int NWT, int S, int MINB>
+template <int NG, int NWR, int NWT, int KC, int S, int MINB>
 __global__ void __launch_bounds__(NWR * NWT * 32, MINB) q4k_q8k_mma_kernel(const q4k_params p) {
   constexpr int RT = NWR, TG = NWT * NG;
-  using ring_t = q4k_ring<RT, TG, Q8K_W, Q8K_X, S>;
+  using ring_t = q4k_ring<RT, TG, Q8K_W, Q8K_X, KC, S>;
+  static_assert(RT == Q8K_W_PACK && TG <= X_PACK_MAX, "one copy per operand");
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const uint32_t smem = smem_u32(smem_raw);
   int* abort_flag = reinterpret_cast<int*>(smem_raw + 120);
@@ -144,25 +151,29 @@ __global__ void __launch_bounds__(NWR * NWT * 32, MINB) q4k_q8k_mma_kernel(const
     const int tr = tile / p.tiles_t, tt = tile - tr * p.tiles_t;
     const int rt = p.rt0 + tr * RT + wr, t0 = (tt * TG + wt * NG) * 8;
     const bool busy = rt < p.rt_end && t0 < p.m;
-    uint64_t acc[NG][8][2];
+    float acc[NG][8][4];
     float accm[NG][4][4];
 #pragma unroll
     for (int g = 0; g < NG; g++) {
 #pragma unroll
-      for (int L = 0; L < 8; L++) acc[g][L][0] = acc[g][L][1] = 0ull;
+      for (int L = 0; L < 8; L++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) acc[g][L][e] = 0.0f;
 #pragma unroll
       for (int e = 0; e < 4; e++)
 #pragma unroll
         for (int k = 0; k < 4; k++) accm[g][e][k] = 0.0f;
     }
-    for (int sb = 0; sb < p.steps; sb++, item++) {
+    for (int ch = 0; ch * KC < p.steps; ch++, item++) {
       const int st = item % S;
       if (!mbar_wait(smem + 8 * st, (item / S) & 1, abort_flag, p.status, 16, item)) return;
-      if (threadIdx.x == 0 && item >= 1) (void)ring.next(p, smem, item - 1 + S, abort_flag);
+      if (threadIdx.x == 0 && item >= 1) ring.next(p, smem, item - 1 + S, abort_flag);
       __syncwarp();
-      if (busy) {
-        const uint8_t* wp = smem_raw + 128 + st * ring_t::STAGE + wr * Q8K_W;
-        const uint8_t* xp = smem_raw + 128 + st * ring_t::STAGE + ring_t::B0 + wt * NG * Q8K_X;
+      const int nb = busy ? min(KC, p.steps - ch * KC) : 0;
+#pragma unroll 1
+      for (int kb = 0; kb < nb; kb++) {
+        const uint8_t* wp = smem_raw + 128 + st * ring_t::STAGE + kb * ring_t::W_STEP + wr * Q8K_W;
+        const uint8_t* xp = smem_raw + 128 + st * ring_t::STAGE + ring_t::B0 + kb * ring_t::X_STEP + wt * NG * Q8K_X;
         const uint2 scp = *reinterpret_cast<const uint2*>(wp + Q8K_W_SC + lane * 8);
         const uint2 dp = *reinterpret_cast<const uint2*>(wp + Q8K_W_D + r * 8);
         const float2 dd0 = __half22float2(*reinterpret_cast<const __half2*>(&dp.x)), dd1 = __half22float2(*reinterpret_cast<const __half2*>(&dp.y));
@@ -176,12 +187,12 @@ __global__ void __launch_bounds__(NWR * NWT * 32, MINB) q4k_q8k_mma_kernel(const
           ol[h] = __hmul2(sl[h], __float2half2_rn(-1024.0f));
           oh[h] = __hmul2(sh[h], __float2half2_rn(-1024.0f));
         }
-        uint64_t s2[NG][2];
+        float sd[NG][4];
 #pragma unroll
         for (int g = 0; g < NG; g++) {
-          const uint64_t dx = *reinterpret_cast<const uint64_t*>(xp + g * Q8K_X + Q8K_X_D + c * 8);
-          s2[g][0] = mul2(pack2(dd0.x, dd0.x), dx);
-          s2[g][1] = mul2(pack2(dd1.x, dd1.x), dx);
+          const float2 dx = *reinterpret_cast<const float2*>(xp + g * Q8K_X + Q8K_X_D + c * 8);
+          sd[g][0] = __fmul_rn(dd0.x, dx.x), sd[g][1] = __fmul_rn(dd0.x, dx.y);
+          sd[g][2] = __fmul_rn(dd1.x, dx.x), sd[g][3] = __fmul_rn(dd1.x, dx.y);
         }
         // The MMAs of lane L are issued before the results of lane L - 1 are used: an MMA takes about 33 cycles, and
         // consecutive ones have to be independent for the tensor pipe to stay busy.
@@ -218,9 +229,8 @@ __global__ void __launch_bounds__(NWR * NWT * 32, MINB) q4k_q8k_mma_kernel(const
           if (L > 0) {
 #pragma unroll
             for (int g = 0; g < NG; g++) {
-              const float* e = d[(L - 1) & 1][g];
-              acc[g][L - 1][0] = fma2(s2[g][0], pack2(e[0], e[1]), acc[g][L - 1][0]);   // mod.rs:759-783
-              acc[g][L - 1][1] = fma2(s2[g][1], pack2(e[2], e[3]), acc[g][L - 1][1]);
+#pragma unroll
+              for (int e = 0; e < 4; e++) acc[g][L - 1][e] = __fmaf_rn(sd[g][e], d[(L - 1) & 1][g][e], acc[g][L - 1][e]);   // mod.rs:759-783
             }
           }
         }
@@ -264,11 +274,7 @@ __global__ void __launch_bounds__(NWR * NWT * 32, MINB) q4k_q8k_mma_kernel(const
       for (int e = 0; e < 4; e++) {
         float v[8];
 #pragma unroll
-        for (int L = 0; L < 8; L++) {
-          float lo, hi;
-          unpack2(acc[g][L][e >> 1], &lo, &hi);
-          v[L] = (e & 1) ? hi : lo;
-        }
+        for (int L = 0; L < 8; L++) v[L] = acc[g][L][e];
         // hsum_ps (dot.rs:447-456), mins (m0+m2)+(m1+m3) (mod.rs:792-794)
         const float s0 = __fadd_rn(v[4], v[0]), s1 = __fadd_rn(v[5], v[1]), s2v = __fadd_rn(v[6], v[2]), s3 = __fadd_rn(v[7], v[3]);
         const float main_val = __fadd_rn(__fadd_rn(s0, s1), __fadd_rn(s2v, s3));
@@ -282,10 +288,11 @@ __global__ void __launch_bounds__(NWR * NWT * 32, MINB) q4k_q8k_mma_kernel(const
 // ---------------------------------------------------------------- dequantize
 
 // Warp tile: 16 WR weight rows x 8 NG activation rows.
-template <int WR, int NG, int NWR, int NWT, int S, int MINB>
+template <int WR, int NG, int NWR, int NWT, int KC, int S, int MINB>
 __global__ void __launch_bounds__(NWR * NWT * 32, MINB) q4k_dequant_mma_kernel(const q4k_params p) {
   constexpr int RT = WR * NWR, TG = NWT * NG;
-  using ring_t = q4k_ring<RT, TG, DEQ_W, DEQ_X, S>;
+  using ring_t = q4k_ring<RT, TG, DEQ_W, DEQ_X, KC, S>;
+  static_assert(RT == DEQ_W_PACK && TG <= X_PACK_MAX, "one copy per operand");
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const uint32_t smem = smem_u32(smem_raw);
   int* abort_flag = reinterpret_cast<int*>(smem_raw + 120);
@@ -310,14 +317,16 @@ __global__ void __launch_bounds__(NWR * NWT * 32, MINB) q4k_dequant_mma_kernel(c
       for (int g = 0; g < NG; g++)
 #pragma unroll
         for (int e = 0; e < 4; e++) acc[i][g][e] = 0.0f;
-    for (int s = 0; s < p.steps; s++, item++) {
+    for (int ch = 0; ch * KC < p.steps; ch++, item++) {
       const int st = item % S;
       if (!mbar_wait(smem + 8 * st, (item / S) & 1, abort_flag, p.status, 17, item)) return;
-      if (threadIdx.x == 0 && item >= 1) (void)ring.next(p, smem, item - 1 + S, abort_flag);
+      if (threadIdx.x == 0 && item >= 1) ring.next(p, smem, item - 1 + S, abort_flag);
       __syncwarp();
-      if (busy) {
-        const uint8_t* wp = smem_raw + 128 + st * ring_t::STAGE + wr * WR * DEQ_W;
-        const uint8_t* xp = smem_raw + 128 + st * ring_t::STAGE + ring_t::B0 + wt * NG * DEQ_X;
+      const int nb = busy ? min(KC, p.steps - ch * KC) : 0;
+#pragma unroll 1
+      for (int kb = 0; kb < nb; kb++) {
+        const uint8_t* wp = smem_raw + 128 + st * ring_t::STAGE + kb * ring_t::W_STEP + wr * WR * DEQ_W;
+        const uint8_t* xp = smem_raw + 128 + st * ring_t::STAGE + ring_t::B0 + kb * ring_t::X_STEP + wt * NG * DEQ_X;
         uint4 wq[WR];
         float4 sc[WR][2];
 #pragma unroll
@@ -415,7 +424,7 @@ __global__ void q4k_build_q8k_kernel(const uint8_t* __restrict__ raw, uint8_t* _
   if (idx >= n_tiles * nb * 32) return;
   const int lane = (int)(idx & 31), r = lane >> 2, c = lane & 3;
   const size_t sb = (idx >> 5) % nb, tile = (idx >> 5) / nb;
-  uint8_t* rec = dst + packed(tile, nb, sb) * Q8K_W;
+  uint8_t* rec = dst + packed(Q8K_W_PACK, tile, nb, sb) * Q8K_W;
   for (int h = 0; h < 2; h++) {
     const size_t row = min(tile * 16 + r + 8 * h, n_rows - 1);
     const uint8_t* blk = raw + (row * nb + sb) * 144;
@@ -437,7 +446,7 @@ __global__ void q4k_build_deq_kernel(const uint8_t* __restrict__ raw, uint8_t* _
   const int lane = (int)(idx & 31), r = lane >> 2, c = lane & 3;
   const size_t grp = (idx >> 5) % (nb * 4), tile = (idx >> 5) / (nb * 4);
   const int g = (int)(grp & 3);
-  uint8_t* rec = dst + packed(tile, nb * 4, grp) * DEQ_W;
+  uint8_t* rec = dst + packed(DEQ_W_PACK, tile, nb * 4, grp) * DEQ_W;
   uint32_t w[2][2];
   for (int h = 0; h < 2; h++) {
     const size_t row = min(tile * 16 + r + 8 * h, n_rows - 1);
@@ -455,7 +464,8 @@ __global__ void q4k_build_deq_kernel(const uint8_t* __restrict__ raw, uint8_t* _
 }
 
 // Q8_K quantizer (mod.rs:82-200) into activation records: one warp per (row, super-block), lane = 8 consecutive values.
-__global__ void __launch_bounds__(256) q8k_records_kernel(const float* __restrict__ x, size_t m, size_t nb, uint8_t* __restrict__ dst) {
+__global__ void __launch_bounds__(256) q8k_records_kernel(const float* __restrict__ x, size_t m, size_t nb, int pack,
+                                                           uint8_t* __restrict__ dst) {
   pdl_wait();
   pdl_launch_dependents();
   const size_t unit = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
@@ -491,7 +501,7 @@ __global__ void __launch_bounds__(256) q8k_records_kernel(const float* __restric
     s += q[i];
   }
   const int n = (int)(t & 7);
-  uint8_t* rec = dst + packed(t >> 3, nb, sb) * Q8K_X;
+  uint8_t* rec = dst + packed(pack, t >> 3, nb, sb) * Q8K_X;
   // values 8 lane ..: group c, low / high half, words 2 (lane % 4), + 1
   const int c = lane >> 3, half = (lane >> 2) & 1;
 #pragma unroll
@@ -510,7 +520,8 @@ __global__ void __launch_bounds__(256) q8k_records_kernel(const float* __restric
 }
 
 // x = p0 + p1 + p2 exactly, bf16 each; one warp per (row, 64-value group), lane = 2 consecutive values.
-__global__ void __launch_bounds__(256) q4k_split_records_kernel(const float* __restrict__ x, size_t m, size_t groups, uint8_t* __restrict__ dst) {
+__global__ void __launch_bounds__(256) q4k_split_records_kernel(const float* __restrict__ x, size_t m, size_t groups, int pack,
+                                                                 uint8_t* __restrict__ dst) {
   pdl_wait();
   pdl_launch_dependents();
   const size_t unit = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
@@ -519,7 +530,7 @@ __global__ void __launch_bounds__(256) q4k_split_records_kernel(const float* __r
   const size_t t = unit / groups, grp = unit - t * groups;
   const float v[2] = {__ldg(x + unit * 64 + lane * 2), __ldg(x + unit * 64 + lane * 2 + 1)};
   const int n = (int)(t & 7), j = lane >> 4;                 // sub-block
-  uint8_t* rec = dst + packed(t >> 3, groups, grp) * DEQ_X;
+  uint8_t* rec = dst + packed(pack, t >> 3, groups, grp) * DEQ_X;
 #pragma unroll
   for (int u = 0; u < 2; u++) {
     const int i = (lane & 15) * 2 + u;                       // value inside the sub-block
@@ -563,45 +574,37 @@ int32_t q4k_mma_launch(rmi_ctx* ctx, K kern, int* cache, int threads, size_t sme
   return rmi_run(ctx, what, kern, dim3((unsigned)(p.n_tiles < slots ? p.n_tiles : slots)), dim3((unsigned)threads), smem, p);
 }
 
-template <int NG, int NWR, int NWT, int S, int MINB>
+template <int NG, int NWR, int NWT, int KC, int S, int MINB>
 int32_t run_q8k(rmi_ctx* ctx, q4k_params p) {
   static int cache[Q4K_MAX_DEVICES];
-  return q4k_mma_launch(ctx, q4k_q8k_mma_kernel<NG, NWR, NWT, S, MINB>, cache, NWR * NWT * 32,
-                        q4k_ring<NWR, NWT * NG, Q8K_W, Q8K_X, S>::SMEM, p, NWR, NWT * NG, "q4k_q8k_mma");
+  return q4k_mma_launch(ctx, q4k_q8k_mma_kernel<NG, NWR, NWT, KC, S, MINB>, cache, NWR * NWT * 32,
+                        q4k_ring<NWR, NWT * NG, Q8K_W, Q8K_X, KC, S>::SMEM, p, NWR, NWT * NG, "q4k_q8k_mma");
 }
-template <int WR, int NG, int NWR, int NWT, int S, int MINB>
+template <int WR, int NG, int NWR, int NWT, int KC, int S, int MINB>
 int32_t run_deq(rmi_ctx* ctx, q4k_params p) {
   static int cache[Q4K_MAX_DEVICES];
-  return q4k_mma_launch(ctx, q4k_dequant_mma_kernel<WR, NG, NWR, NWT, S, MINB>, cache, NWR * NWT * 32,
-                        q4k_ring<WR * NWR, NWT * NG, DEQ_W, DEQ_X, S>::SMEM, p, WR * NWR, NWT * NG, "q4k_dequant_mma");
+  return q4k_mma_launch(ctx, q4k_dequant_mma_kernel<WR, NG, NWR, NWT, KC, S, MINB>, cache, NWR * NWT * 32,
+                        q4k_ring<WR * NWR, NWT * NG, DEQ_W, DEQ_X, KC, S>::SMEM, p, WR * NWR, NWT * NG, "q4k_dequant_mma");
 }
 
-int32_t build_records(rmi_ctx* ctx, const rmi_weight* cw, bool deq) {
-  rmi_weight* w = const_cast<rmi_weight*>(cw);
-  uint8_t*& slot = deq ? w->d_q4k_deq : w->d_q4k_q8k;
-  if (slot != nullptr) return RMI_OK;
-  const size_t nb = w->n_in / 256, n_tiles = (w->n_tiles16 + PACK - 1) / PACK * PACK, recs = n_tiles * nb * (deq ? 4 : 1);
+int32_t build_records(rmi_ctx* ctx, rmi_weight* w, bool deq) {
+  const size_t nb = w->n_in / 256, pack = deq ? DEQ_W_PACK : Q8K_W_PACK;
+  const size_t n_tiles = (w->n_tiles16 + pack - 1) / pack * pack, recs = n_tiles * nb * (deq ? 4 : 1);
   const size_t bytes = recs * (deq ? DEQ_W : Q8K_W);
   uint8_t* d = nullptr;
   if (cudaMalloc((void**)&d, bytes) != cudaSuccess) {
     (void)cudaGetLastError();
-    rmi_set_error("device allocation of %zu bytes failed", bytes);
     return RMI_ERR_OOM;
   }
   const unsigned grid = (unsigned)((recs * 32 + 255) / 256);
   if (deq) q4k_build_deq_kernel<<<grid, 256, 0, ctx->stream>>>(w->d_raw, d, w->n_rows, n_tiles, nb);
   else q4k_build_q8k_kernel<<<grid, 256, 0, ctx->stream>>>(w->d_raw, d, w->n_rows, n_tiles, nb);
-  int32_t st = rmi_post_launch(ctx, "q4k_build_records");
   // complete before any kernel of a dependent launch may fetch it ahead of its wait
-  if (st == RMI_OK && cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
-    rmi_set_error("weight re-layout failed: %s", cudaGetErrorString(cudaGetLastError()));
-    st = RMI_ERR_CUDA;
-  }
-  if (st != RMI_OK) {
+  if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
     cudaFree(d);
-    return st;
+    return RMI_ERR_CUDA;
   }
-  slot = d;
+  (deq ? w->d_q4k_deq : w->d_q4k_q8k) = d;
   w->frag_bytes += bytes;
   return RMI_OK;
 }
@@ -621,35 +624,50 @@ q4k_params base_params(rmi_ctx* ctx, const rmi_weight* w, const uint8_t* x, size
 
 }  // namespace
 
+// The records are built on first use.  False inside a stream capture, or without memory for them.
+bool q4k_mma_prepare(rmi_ctx* ctx, const rmi_weight* w, bool dequant) {
+  if ((dequant ? w->d_q4k_deq : w->d_q4k_q8k) != nullptr) return true;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return build_records(ctx, const_cast<rmi_weight*>(w), dequant) == RMI_OK;
+}
+
 size_t q4k_mma_x_bytes(const rmi_weight* w, size_t m, bool dequant) {
-  const size_t nb = w->n_in / 256, groups = (m + 8 * PACK - 1) / (8 * PACK) * PACK;
+  const size_t nb = w->n_in / 256, groups = (m + 8 * X_PACK_MAX - 1) / (8 * X_PACK_MAX) * X_PACK_MAX;
   return dequant ? groups * nb * 4 * DEQ_X : groups * nb * Q8K_X;
 }
 
-// AVX2 order; x f32 rows, xrec scratch of q4k_mma_x_bytes
+// AVX2 order; q4k_mma_prepare succeeded; x f32 rows, xrec scratch of q4k_mma_x_bytes
 int32_t launch_q4k_q8k_mma(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, uint8_t* xrec, float* out, size_t row_begin,
                            size_t row_end) {
   if (m == 0 || row_begin >= row_end) return RMI_OK;
-  RMI_TRY(build_records(ctx, w, false));
+  // 16 activation rows per CTA (the conversion of the nibbles is shared by two MMA column tiles); 8 where that leaves half
+  // of the SMs without work (16 rows of 4096 x 4096: 12.0 -> 7.8 us)
+  const size_t packs = (row_end + 16 * Q8K_W_PACK - 1) / (16 * Q8K_W_PACK) - row_begin / (16 * Q8K_W_PACK);
+  const int groups = packs * ((m + 15) / 16) * 2 <= (size_t)ctx->sm_count ? 1 : 2;
   const size_t nb = w->n_in / 256, warps = m * nb;
-  RMI_TRY(rmi_run(ctx, "q8k_records", q8k_records_kernel, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, x, m, nb, xrec));
+  RMI_TRY(rmi_run(ctx, "q8k_records", q8k_records_kernel, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, x, m, nb, groups, xrec));
   q4k_params p = base_params(ctx, w, xrec, m, out);
   p.w = w->d_q4k_q8k;
   p.steps = (int)nb;
-  p.rt0 = (int)(row_begin / (16 * PACK)) * PACK;
+  p.rt0 = (int)(row_begin / (16 * Q8K_W_PACK)) * Q8K_W_PACK;
   p.rt_end = (int)((row_end + 15) / 16);
   p.row_begin = (int)row_begin;
   p.row_end = (int)row_end;
-  return run_q8k<2, 4, 2, 3, 1>(ctx, p);
+  return groups == 1 ? run_q8k<1, 4, 1, 4, 2, 3>(ctx, p) : run_q8k<2, 4, 1, 3, 2, 2>(ctx, p);
 }
 
 int32_t launch_q4k_dequant_mma(rmi_ctx* ctx, const rmi_weight* w, const float* x, size_t m, uint8_t* xrec, float* out) {
   if (m == 0 || w->n_rows == 0) return RMI_OK;
-  RMI_TRY(build_records(ctx, w, true));
+  // 16 activation rows per CTA, 8 while that leaves SMs without work (16 rows of 4096 x 4096: 28.9 -> 22.6 us, 48: 43 -> 36)
+  const int tg = (w->n_tiles16 + DEQ_W_PACK - 1) / DEQ_W_PACK * ((m + 15) / 16) <= (size_t)ctx->sm_count ? 1 : 2;
   const size_t groups = w->n_in / 64, warps = m * groups;
-  RMI_TRY(rmi_run(ctx, "q4k_split_records", q4k_split_records_kernel, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, x, m, groups, xrec));
+  RMI_TRY(rmi_run(ctx, "q4k_split_records", q4k_split_records_kernel, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, x, m, groups, tg, xrec));
   q4k_params p = base_params(ctx, w, xrec, m, out);
   p.w = w->d_q4k_deq;
   p.steps = (int)groups;
-  return run_deq<1, 2, 4, 2, 4, 2>(ctx, p);
+  return tg == 1 ? run_deq<2, 1, 4, 1, 4, 2, 3>(ctx, p) : run_deq<2, 2, 4, 1, 4, 2, 2>(ctx, p);
 }

@@ -87,3 +87,24 @@ def test_prefill_attention_rows_and_heads(rmi, ctx, tmp_path, head_dim, n_head, 
         assert np.array_equal(loop, batched)
     s.free()
     model.free()
+
+
+# Q4_K on the tensor cores: the fewest rows, both CTA widths, rows and super-blocks that fill no tile, chunk or ring
+@pytest.mark.parametrize("m,n,k", [(3, 5, 256), (9, 130, 512), (16, 1030, 1280), (33, 2600, 768), (5, 8200, 256), (200, 777, 2304)])
+def test_q4_k_on_tensor_cores(rmi, ctx, m, n, k):
+    torch = pytest.importorskip("torch")
+    wb = rmi.synth.q4_k_weight(n, k, seed=m + n)
+    w = rmi.QuantizedTensor.from_bytes(wb, rmi.GGML_Q4_K, k, n)
+    x = rmi.synth.normal((m, k), seed=k)
+    x[m // 2, : k // 2] = 0.0
+    d, out = torch.from_numpy(x).cuda(), torch.empty((m, n), device="cuda")
+    torch.cuda.synchronize()
+    rmi.matmul_q4_k_q8k_dev(w, d.data_ptr(), m, out.data_ptr())
+    ctx.sync()
+    ref = np.stack([orc.q4k_forward_prepared(wb, x[t], k, n) for t in range(m)])
+    assert np.array_equal(bits(out.cpu().numpy()), bits(ref))
+    rmi.matmul_q4_k_dequant_dev(w, d.data_ptr(), m, out.data_ptr())
+    ctx.sync()
+    ref = x.astype(np.float64) @ orc.dequantize_q4_k_weight(wb, n, k).astype(np.float64).T
+    assert rel_err(out.cpu().numpy(), ref.astype(np.float32)) < 2e-6     # no input is rounded, sums are f32
+    w.free()
