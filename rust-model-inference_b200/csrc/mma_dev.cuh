@@ -1,5 +1,4 @@
-// Device helpers of the warp-level tensor-core matmuls: bounded mbarrier waits, bulk copies, warp-level MMA, packed
-// f32 arithmetic.
+// Device helpers of the warp-level tensor-core matmuls: bounded mbarrier waits, bulk copies, warp-level MMA.
 #pragma once
 #include <cuda_bf16.h>
 
@@ -69,31 +68,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
                                           int site, int detail) {
   if (mbar_try(bar, parity)) return true;
   return mbar_wait_slow(bar, parity, abort_flag, status, site, detail);
-}
-
-// ---- packed f32x2 arithmetic (two independent IEEE round-to-nearest operations) ----
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float* lo, float* hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(*lo), "=f"(*hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
 }
 
 // ---- warp-level MMA: D[16x8] (+)= A[16xK] B[Kx8], f32 result ----
